@@ -22,6 +22,7 @@
 #include "guide.h"
 #include "layout.h"
 #include "refit.h"
+#include "wide_build.h"
 
 static_assert(sizeof(tc_gpu_render_params) == 96, "GpuRenderParams is 96 bytes");
 static_assert(sizeof(tc_gpu_camera) == 64, "GpuCamera is 64 bytes");
@@ -96,6 +97,8 @@ struct tc_context {
   uint32_t sphere_count = 0, triangle_count = 0, material_count = 0, light_count = 0, bvh_prims = 0;
   uint32_t bvh_depth = 0;
   size_t pair_count = 0;
+  // Four-wide form of the hierarchy (wide_build.cu), rewritten whenever the hierarchy changes.
+  DevBuf wide_nodes, wide_leaves, wide_scan;
   bool any_attr = false;
   // Geometry refit (tc_update_geometry): the root record, the scene-order geometry the prim
   // records are rewritten from, and pair-node indices grouped by depth.
@@ -336,6 +339,30 @@ int check_render_params(tc_context* ctx, const tc_gpu_render_params* p) {
   return TC_OK;
 }
 
+// Sizes the buffers of the four-wide form of a hierarchy of `pairs` interior nodes over `prims`
+// primitives. Leaves the scene without one (scene.wide null: the pair traversal) when a node index
+// would not fit the traversal's 32-bit byte offsets or its stack.
+int reserve_wide(tc_context* ctx, size_t prims, size_t pairs, uint32_t depth) {
+  ctx->scene.wide = nullptr;
+  ctx->scene.leaves = nullptr;
+  if (pairs > tcb::kMaxWideNodes || depth > tcb::kMaxWideDepth || prims == 0) return TC_OK;
+  TC_CUDA(ctx, ctx->wide_nodes.reserve(sizeof(tcb::WideNode) * std::max<size_t>(pairs, 1)));
+  TC_CUDA(ctx, ctx->wide_leaves.reserve(sizeof(tcb::LeafPair) * tcb::max_leaf_pairs(prims, pairs)));
+  TC_CUDA(ctx, ctx->wide_scan.reserve(sizeof(uint32_t) * tcb::wide_scan_words(prims)));
+  ctx->scene.wide = ctx->wide_nodes.as<tcb::WideNode>();
+  ctx->scene.leaves = ctx->wide_leaves.as<tcb::LeafPair>();
+  return TC_OK;
+}
+
+// Writes the four-wide form of the hierarchy now in ctx->pairs and ctx->prims (when it has one).
+int build_wide(tc_context* ctx, uint32_t prims, uint32_t pairs, cudaStream_t st) {
+  if (!ctx->scene.wide) return TC_OK;
+  TC_CUDA(ctx, tcb::launch_wide_build(ctx->pairs.as<tcb::PairNode>(), pairs, ctx->prims.as<tcb::PrimRecord>(), prims,
+                                      ctx->wide_scan.as<uint32_t>(), ctx->wide_nodes.as<tcb::WideNode>(),
+                                      ctx->wide_leaves.as<tcb::LeafPair>(), st));
+  return TC_OK;
+}
+
 // Device hierarchy of a scene: the caller's flat BVH in the reference layout (when given and
 // use_given is set) or a fresh median-split build (crates/toaster-bvh/src/bvh.rs:92-154).
 int build_hierarchy(tc_context* ctx, const tc_scene_data* sd, bool use_given, tcb::DeviceHierarchy& dh) {
@@ -544,7 +571,7 @@ int tc_upload_scene(tc_context* ctx, const tc_scene_data* sd) {
   const size_t n_prims = sd->sphere_count + sd->triangle_count;
   const bool given = sd->bvh_nodes && sd->bvh_node_count;
   const bool on_device = !given && (ctx->build_mode == 2 || (ctx->build_mode == 0 && n_prims >= kDeviceBuildMin));
-  bool built = false;
+  bool built = false, unions = true;
   uint32_t pair_count = 0, prim_count = 0, depth = 0;
   if (on_device) {
     TC_CUDA(ctx, ctx->builder.plan(uint32_t(sd->sphere_count), uint32_t(sd->triangle_count)));
@@ -585,6 +612,7 @@ int tc_upload_scene(tc_context* ctx, const tc_scene_data* sd) {
   if (!built) {
     tcb::DeviceHierarchy dh;
     if (int rc = build_hierarchy(ctx, sd, true, dh)) return rc;
+    if (given) unions = tcb::bounds_are_unions(dh);
     TC_CUDA(ctx, upload(ctx->pairs, dh.pairs.data(), dh.pairs.size(), st));
     TC_CUDA(ctx, upload(ctx->prims, dh.prims.data(), dh.prims.size(), st));
     TC_CUDA(ctx, upload(ctx->root_buf, &dh.root, 1, st));
@@ -619,6 +647,10 @@ int tc_upload_scene(tc_context* ctx, const tc_scene_data* sd) {
   s.pairs = ctx->pairs.as<tcb::PairNode>();
   s.prims = ctx->prims.as<tcb::PrimRecord>();
   s.root = ctx->root_buf.as<tcb::ChildRec>();
+  if (unions) {
+    if (int rc = reserve_wide(ctx, prim_count, pair_count, depth)) return rc;
+    if (int rc = build_wide(ctx, prim_count, pair_count, st)) return rc;
+  }
   s.materials = ctx->materials.as<tcb::DevMaterial>();
   s.material_count = n_mat;
   s.lights = sd->light_count ? ctx->lights.as<tcb::DevLight>() : nullptr;
@@ -747,6 +779,7 @@ int tc_update_geometry(tc_context* ctx, const tc_scene_data* sd, const tc_scene_
     TC_CUDA(ctx, tcb::launch_refit(plan, ctx->pairs.as<tcb::PairNode>(), ctx->root_buf.as<tcb::ChildRec>(),
                                    ctx->prims.as<tcb::PrimRecord>(), ctx->bvh_prims,
                                    ctx->raw_spheres.as<tc_gpu_sphere>(), ctx->raw_triangles.as<tc_gpu_triangle>(), st));
+    if (int rc = build_wide(ctx, ctx->bvh_prims, uint32_t(ctx->pair_count), st)) return rc;
     if (ctx->scene.tri_verts && changes->triangles)
       TC_CUDA(ctx, tcb::launch_triangle_vertices(ctx->prims.as<tcb::PrimRecord>(), ctx->bvh_prims,
                                                  ctx->raw_triangles.ptr, ctx->tri_verts.as<float4>(), st));
@@ -1532,6 +1565,8 @@ static int animation_enqueue(tc_animation* a, cudaStream_t st) {
                                    ctx->prims.as<tcb::PrimRecord>(), ctx->bvh_prims,
                                    ctx->raw_spheres.as<tc_gpu_sphere>(), ctx->raw_triangles.as<tc_gpu_triangle>(), st));
   }
+  if (int rc = build_wide(ctx, ctx->bvh_prims, a->rebuild ? ctx->builder.pair_count() : uint32_t(ctx->pair_count), st))
+    return rc;
   const float* cam = a->d_frame.as<float>();
   const uint32_t* fi = reinterpret_cast<const uint32_t*>(cam + 16);
   if (int rc = enqueue_render(ctx, &a->params, a->options, st, false, fi, cam, a->h_counters)) return rc;
@@ -1577,6 +1612,14 @@ int tc_animation_create(tc_context* ctx, const tc_scene_data* first_frame, const
     if (e == cudaSuccess) e = ctx->builder.plan(ctx->sphere_count, ctx->triangle_count);
     if (e == cudaSuccess)
       e = ctx->pairs.reserve(sizeof(tcb::PairNode) * std::max<size_t>(ctx->builder.pair_count(), 1));
+    if (e == cudaSuccess) {
+      // The first frame below builds into these buffers; until then the scene has no wide form.
+      ctx->scene.pairs = ctx->pairs.as<tcb::PairNode>();
+      if (int rc = reserve_wide(ctx, ctx->bvh_prims, ctx->builder.pair_count(), ctx->builder.depth())) {
+        animation_free(a);
+        return rc;
+      }
+    }
     if (e == cudaSuccess) e = ctx->build_status.reserve(sizeof(uint32_t));
     if (e == cudaSuccess && a->h_attr_flags) e = ctx->attr_flags.reserve(sizeof(uint32_t) * ctx->triangle_count);
   }
@@ -1589,6 +1632,7 @@ int tc_animation_create(tc_context* ctx, const tc_scene_data* first_frame, const
   if (e == cudaSuccess && ctx->triangle_count)
     e = ctx->raw_triangles.reserve(sizeof(tc_gpu_triangle) * ctx->triangle_count);
   if (e != cudaSuccess) {
+    if (a->rebuild) ctx->scene.wide = nullptr;
     animation_free(a);
     return cuda_fail(ctx, e, "animation buffers");
   }

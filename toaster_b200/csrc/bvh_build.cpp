@@ -294,4 +294,18 @@ bool to_device_layout(const FlatHierarchy& flat, const SphereIn* spheres, const 
   return true;
 }
 
+bool bounds_are_unions(const DeviceHierarchy& h) {
+  auto ok = [&](const ChildRec& c) {
+    if (c.link & kLeafBit) return true;
+    const ChildRec& l = h.pairs[c.link].child[0];
+    const ChildRec& r = h.pairs[c.link].child[1];
+    return c.min_x == std::min(l.min_x, r.min_x) && c.min_y == std::min(l.min_y, r.min_y) &&
+           c.min_z == std::min(l.min_z, r.min_z) && c.max_x == std::max(l.max_x, r.max_x) &&
+           c.max_y == std::max(l.max_y, r.max_y) && c.max_z == std::max(l.max_z, r.max_z);
+  };
+  for (const PairNode& p : h.pairs)
+    if (!ok(p.child[0]) || !ok(p.child[1])) return false;
+  return ok(h.root);
+}
+
 }  // namespace tcb

@@ -61,6 +61,11 @@ bool to_device_layout(const FlatHierarchy& flat, const SphereIn* spheres, const 
                       const uint32_t* triangle_attr_flags, size_t n_triangles, DeviceHierarchy& out,
                       std::string& error);
 
+// Whether every interior node's box is the union of its children's, as every built or refitted
+// hierarchy's is; a caller's own may not be, and then has no four-wide form (traverse_wide.cuh
+// reconstructs an interior box's entry distance from its children's planes).
+bool bounds_are_unions(const DeviceHierarchy& h);
+
 }  // namespace tcb
 
 #endif

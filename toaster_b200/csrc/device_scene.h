@@ -12,6 +12,9 @@ namespace tcb {
 
 struct DevScene {
   const PairNode* pairs;
+  // Four-wide form of the hierarchy (wide_build.cu), or null when it has none (see there).
+  const WideNode* wide;
+  const LeafPair* leaves;
   const PrimRecord* prims;
   const ChildRec* root;  // device memory: the root's bounds and link
   const DevMaterial* materials;

@@ -6,7 +6,10 @@
 //                         the FP64 sums, new camera paths in free slots
 //   wf_shade_kernel       wavefront schedule: the material queues in order (BSDF, light and
 //                         environment NEE, the next ray), guided or recording when asked
-//   wf_trace_kernel       wavefront schedule: extension rays then shadow rays, 32 per warp
+//   wf_trace_wide_kernel  wavefront schedule: extension rays then shadow rays through the four-wide
+//                         hierarchy, finished lanes refilled from the queue
+//   wf_trace_kernel       the same over the binary hierarchy, 32 rays per warp (watertight triangle
+//                         test, ray sorting, refill option, hierarchies without a four-wide form)
 //   wf_sort_* kernels     optional ray sorting before tracing (kind, octant, origin bucket)
 //   render_kernel         persistent path-tracing megakernel (small frames, batched launches,
 //                         captured animation frames)
@@ -32,6 +35,7 @@
 #include "device_scene.h"
 #include "guide.h"
 #include "traverse.cuh"
+#include "traverse_wide.cuh"
 
 namespace tcb {
 
@@ -1638,6 +1642,68 @@ __global__ void __launch_bounds__(128) wf_trace_kernel(const WavefrontLaunch W) 
   if (threadIdx.x < 2 && s_count[threadIdx.x] != 0ull) atomicAdd(W.r.counters + 1 + threadIdx.x, s_count[threadIdx.x]);
 }
 
+// The default trace launch: four-wide traversal (traverse_wide.cuh) with lane refills. A warp takes
+// queue entries for its idle lanes (one atomic) as soon as no more than kTraceRefill lanes still
+// traverse; 16 / 20 / 24 took 26.4 / 26.1 / 26.2 ms in the room and 7.7 / 7.8 / 8.1 ms on the terrain.
+// Eight blocks per SM (64 registers) took 9.2 / 24.9 / 7.7 ms on the mixed scene, the room and the
+// terrain, seven 9.5 / 25.3 / 7.9 ms; nine and ten spill (10.8 / 30.8 / 9.0 ms at nine).
+constexpr int kTraceBlock = 128;
+constexpr int kTraceRefill = 20;
+__global__ void __launch_bounds__(kTraceBlock, 8) wf_trace_wide_kernel(const __grid_constant__ WavefrontLaunch W) {
+  __shared__ ChildRec root;
+  __shared__ float s_dir[3 * kTraceBlock];
+  __shared__ uint32_t s_entry[kTraceBlock], s_target[kTraceBlock];  // queue entry of the lane's ray, its target
+  float* const dir = s_dir + threadIdx.x;
+  const DevScene& s = W.r.f.scene;
+  const uint32_t n_ext = W.q[kWfExtCount], total = n_ext + W.q[kWfShadowCount];
+  if (threadIdx.x == 0) {
+    root = *s.root;
+    if (blockIdx.x == 0) {  // every queued ray is traced exactly once
+      if (n_ext) atomicAdd(W.r.counters + 1, (unsigned long long)n_ext);
+      if (total > n_ext) atomicAdd(W.r.counters + 2, (unsigned long long)(total - n_ext));
+    }
+  }
+  s_entry[threadIdx.x] = kNoNode;
+  __syncthreads();
+  bool any_hit = false, exhausted = false;
+  WideRay w;
+  WideTraversal T;
+  T.cur = kNoNode;
+  uint2 st[kMaxStack];
+  for (;;) {
+    const unsigned live = __ballot_sync(0xffffffffu, T.live());
+    if (live == 0u || (!exhausted && __popc(live) <= kTraceRefill)) {
+      if (!T.live() && s_entry[threadIdx.x] != kNoNode) {
+        const bool hit = T.rec != kNoNode;
+        const uint32_t tag = hit && !any_hit ? __float_as_uint(__ldg(&s.prims[T.rec].a[3])) : 0u;
+        wf_entry_result(W, s_entry[threadIdx.x], n_ext, s_target[threadIdx.x], hit, T.closest, T.rec, tag);
+        s_entry[threadIdx.x] = kNoNode;
+      }
+      if (exhausted) break;
+      const uint32_t want = 32u - uint32_t(__popc(live));
+      uint32_t first = 0;
+      if ((threadIdx.x & 31u) == 0u) first = atomicAdd(W.q + kWfTraceCursor, want);
+      first = __shfl_sync(0xffffffffu, first, 0);
+      exhausted = first + want >= total;
+      const uint32_t i = first + uint32_t(__popc(~live & lanes_below()));
+      if (!T.live() && i < total) {
+        float tmax;
+        uint32_t target;
+        const RayQ q = wf_entry_ray<false>(W, i, n_ext, tmax, target);
+        s_entry[threadIdx.x] = i;
+        s_target[threadIdx.x] = target;
+        any_hit = i >= n_ext;
+        w = make_wide_ray(q);
+        store_direction<kTraceBlock>(dir, q);
+        wide_begin(T, s.pairs, s.prims, s.root, root, q, kRayEps, tmax, any_hit);
+      }
+    }
+    // Once the queue is empty the node phase ends when half of the remaining lanes have left it.
+    const int left = __popc(__ballot_sync(0xffffffffu, T.live()));
+    wide_round<kTraceBlock>(T, w, dir, kRayEps, any_hit, s.wide, s.leaves, st, exhausted ? left >> 1 : kNodeKeep);
+  }
+}
+
 // Counting sort of one iteration's queued rays by key (extension entries 0..n_ext, then shadow
 // entries): block b of kWfSortBlocks counts the keys of its contiguous share of the entries in
 // shared memory and stores its counts bin-major; a one-block scan turns the counts into each
@@ -1714,6 +1780,7 @@ cudaError_t launch_wavefront_iteration(const WavefrontLaunch& w, bool moments, i
   static const int shade_per_sm = resident_blocks(wf_shade_kernel<false>, 128);
   static const int guided_shade_per_sm = resident_blocks(wf_shade_kernel<true>, 128);
   static const int trace_per_sm = resident_blocks(wf_trace_kernel<false, false, false>, 128);
+  static const int wide_per_sm = resident_blocks(wf_trace_wide_kernel, kTraceBlock);
   static const int sorted_per_sm = resident_blocks(wf_trace_kernel<false, false, true>, 128);
   static const int refill_per_sm = resident_blocks(wf_trace_kernel<true, false, false>, 128);
   static const int watertight_per_sm = resident_blocks(wf_trace_kernel<false, true, false>, 128);
@@ -1751,6 +1818,8 @@ cudaError_t launch_wavefront_iteration(const WavefrontLaunch& w, bool moments, i
     wf_trace_kernel<false, true, false><<<watertight_per_sm * sm_count, 128, 0, stream>>>(w);
   } else if (w.refill_lanes > 1) {
     wf_trace_kernel<true, false, false><<<refill_per_sm * sm_count, 128, 0, stream>>>(w);
+  } else if (w.r.f.scene.wide) {
+    wf_trace_wide_kernel<<<wide_per_sm * sm_count, kTraceBlock, 0, stream>>>(w);
   } else {
     wf_trace_kernel<false, false, false><<<trace_per_sm * sm_count, 128, 0, stream>>>(w);
   }

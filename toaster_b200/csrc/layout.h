@@ -48,6 +48,37 @@ struct alignas(16) PairNode {
 };
 static_assert(sizeof(PairNode) == 64, "PairNode is 64 bytes");
 
+// Four-wide form of the same hierarchy for the main traversal (traverse_wide.cuh).
+//
+// A wide node holds the children of a pair's two children (a child that is a leaf takes the first
+// slot of its half and leaves the other empty): slots 0-1 come from child 0, slots 2-3 from child
+// 1. Each quad holds one plane of the four boxes: quads 0-5 = lo x, hi x, lo y, hi y, lo z, hi z,
+// quad 6 = links (pair index, which is the wide node's too, or kLeafBit | first LeafPair). Quad f of
+// node i is stored at position f ^ (i & 7): the lanes of a warp read the same quad of unrelated
+// nodes, and without the swizzle those addresses would all fall into the same eighth of the L1 banks.
+struct alignas(128) WideNode {
+  uint32_t quad[8][4];
+};
+static_assert(sizeof(WideNode) == 128, "WideNode is one 128-byte line");
+constexpr uint32_t kMaxWideNodes = 1u << 25;  // traversal addresses nodes with 32-bit byte offsets
+constexpr uint32_t kMaxWideDepth = 42;        // three entries per two levels fit kMaxStack
+
+// Two consecutive primitives of one leaf, component by component, so that one packed operation
+// serves both: -v0x -v0y -v0z e1x | e1y e1z e2x -e2y | -e2z, first record and flags (each component
+// twice, primitive 0 then 1; the flipped signs make every sum of products in the triangle test a
+// difference). Spheres: v0 = centre, e1x = radius, e1y = radius^2. A missing second primitive is all
+// zero: its determinant is 0, so it is never hit.
+struct alignas(32) LeafPair {
+  float nv0x[2], nv0y[2], nv0z[2], e1x[2], e1y[2], e1z[2], e2x[2], ne2y[2], ne2z[2];
+  uint32_t first;  // PrimRecord index of primitive 0
+  uint32_t flags;
+  uint32_t unused[4];
+};
+static_assert(sizeof(LeafPair) == 96, "LeafPair is three 32-byte sectors");
+constexpr uint32_t kPairLast = 1u;     // last pair of its leaf
+constexpr uint32_t kPairSphere0 = 2u;  // primitive 0 / 1 is a sphere
+constexpr uint32_t kPairSphere1 = 4u;
+
 struct alignas(16) PrimRecord {
   float a[4];
   float b[4];
