@@ -9,6 +9,7 @@ is one path's radiance, the images must be equal exactly.
 import numpy as np
 import pytest
 
+import oracle
 from toaster_b200 import configs, gpu_types as gt, native
 from toaster_b200.scene import EnvironmentMap, Material, Scene, scene_to_gpu
 
@@ -74,3 +75,18 @@ def test_given_hierarchies(renderer, loosened):
         nodes["max"][interior[1], :3] += np.float32(0.25)
     renderer.upload(scene_to_gpu(scene_of(300, 10, 3), bvh=(nodes, refs)))
     assert_same_image(renderer)
+
+
+# Ray counts around every change of the launch: one lane per warp, each power of two up to full
+# warps, partial last pieces, more rays than one resident wave holds lanes.
+@pytest.mark.parametrize("count", [1, 3, 31, 33, 127, 2368, 2369, 4737, 9473, 18945, 37889, 75777, 200003, 400001])
+def test_hits_at_every_launch_shape(renderer, count):
+    scene = scene_of(1500, 40, 9)
+    rays = configs.parity_rays(scene, count, seed=count)
+    rays[::7, 4] = 0.0  # axis-parallel components go to the pair traversal
+    rays[::11, 3] = -0.0
+    renderer.upload(scene_to_gpu(scene))
+    prim, t = renderer.trace_closest(rays)
+    want_prim, want_t = oracle.Oracle(scene).trace_closest(rays)
+    assert np.array_equal(prim, want_prim)
+    assert np.array_equal(t.view(np.uint32)[prim != 0xFFFFFFFF], want_t.view(np.uint32)[prim != 0xFFFFFFFF])

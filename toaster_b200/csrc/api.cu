@@ -1863,7 +1863,7 @@ int tc_trace_closest_device_async(tc_context* ctx, const float* d_rays, size_t n
   if (n && (!d_rays || !d_prim || !d_t)) return fail(ctx, TC_ERR_INVALID, "ray or output pointer is null");
   TC_CUDA(ctx, cudaSetDevice(ctx->device));
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
-  TC_CUDA(ctx, tcb::launch_trace_closest(ctx->scene, d_rays, n, tmin, d_prim, d_t, st));
+  TC_CUDA(ctx, tcb::launch_trace_closest(ctx->scene, d_rays, n, tmin, d_prim, d_t, ctx->sm_count, st));
   return TC_OK;
 }
 
@@ -1881,7 +1881,7 @@ int tc_trace_closest(tc_context* ctx, const float* rays, size_t n, float tmin, u
   TC_CUDA(ctx, cudaMemcpyAsync(ctx->ray_buf.ptr, rays, sizeof(float) * 6 * n, cudaMemcpyHostToDevice, st));
   TC_CUDA(ctx, cudaEventRecord(ctx->ev_kernel0, st));
   TC_CUDA(ctx, tcb::launch_trace_closest(ctx->scene, ctx->ray_buf.as<float>(), n, tmin, ctx->prim_buf.as<uint32_t>(),
-                                         ctx->t_buf.as<float>(), st));
+                                         ctx->t_buf.as<float>(), ctx->sm_count, st));
   TC_CUDA(ctx, cudaEventRecord(ctx->ev_kernel1, st));
   TC_CUDA(ctx, cudaMemcpyAsync(prim, ctx->prim_buf.ptr, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, st));
   TC_CUDA(ctx, cudaMemcpyAsync(t, ctx->t_buf.ptr, sizeof(float) * n, cudaMemcpyDeviceToHost, st));

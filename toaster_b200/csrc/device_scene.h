@@ -178,7 +178,7 @@ cudaError_t launch_triangle_vertices(const PrimRecord* prims, uint32_t n, const 
 
 // Launchers implemented in kernels.cu. All enqueue on `stream` and return the launch error.
 cudaError_t launch_trace_closest(const DevScene& s, const float* rays, uint64_t n, float tmin, uint32_t* prim,
-                                 float* t, cudaStream_t stream);
+                                 float* t, int sm_count, cudaStream_t stream);
 cudaError_t launch_render(const RenderLaunch& r, int block_size, int grid_size, bool moments, cudaStream_t stream,
                           int mode = kModePlain);
 int render_max_blocks_per_sm(int block_size, bool moments, int mode = kModePlain, int short_stack = 0,

@@ -1,6 +1,8 @@
 // CUDA kernels of the toaster B200 path tracer (sm_100a).
 //
-//   trace_closest_kernel  closest-hit parity hook: one ray per thread, exact traversal
+//   trace_closest_wide_kernel  closest-hit queries through the four-wide hierarchy
+//   trace_closest_kernel  the same, one ray per thread over the sibling pairs (watertight triangle
+//                         test, hierarchies without a four-wide form)
 //   wf_logic_kernel       wavefront schedule, one slot per thread: shadow-ray results, the last
 //                         hit (miss, emission or the slot's material queue), finished paths into
 //                         the FP64 sums, new camera paths in free slots
@@ -232,6 +234,14 @@ __device__ __forceinline__ float power_heuristic(float a, float b) {
   return d > 0.0f ? a2 / d : 0.0f;
 }
 
+// Resident blocks per SM of a kernel at a block size.
+template <class K>
+static int resident_blocks(K kernel, int block) {
+  int blocks = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, block, 0) != cudaSuccess) return 1;
+  return blocks > 0 ? blocks : 1;
+}
+
 // ------------------------------------------------------------------------ parity kernel
 __global__ void trace_closest_kernel(const DevScene s, const float* __restrict__ rays, uint64_t n, float tmin,
                                      uint32_t* __restrict__ prim, float* __restrict__ tout) {
@@ -249,6 +259,76 @@ __global__ void trace_closest_kernel(const DevScene s, const float* __restrict__
                        : trace_ray(s.pairs, s.prims, root, q, tmin, CUDART_INF_F, false, tr, visits);
   prim[i] = hit ? (tr.tag & ~kTagLast) : 0xFFFFFFFFu;
   tout[i] = hit ? tr.t : CUDART_INF_F;
+}
+
+// Closest hits through the four-wide hierarchy. The rays are dealt to the blocks in pieces of
+// 2^width_log2 consecutive rays, piece p to block p mod gridDim.x, so every block gets the same mix of
+// cheap and expensive rays and one resident wave does the call; a block's warps take its rays from a
+// cursor in shared memory as lanes fall idle. Only the first 2^width_log2 lanes of a warp take
+// rays: when there are too few rays to fill the GPU, fewer per warp keep more warps busy and leave
+// each with less divergence. One million rays: 443 -> 276 us (2,051 primitives), 350 -> 235 (mixed
+// scene), 1,450 -> 904 (room), 432 -> 301 (terrain of 2.1 M triangles), against one thread per ray
+// over the pairs; 65,536 rays: 76 -> 68, 68 -> 65, 214 -> 157 and 93 -> 73; 4,096 rays: 74 -> 49,
+// 64 -> 38, 199 -> 98 and 64 -> 41 us.
+constexpr int kHitsBlock = 128;
+__global__ void __launch_bounds__(kHitsBlock, 8)
+    trace_closest_wide_kernel(const __grid_constant__ DevScene s, const float* __restrict__ rays, uint64_t n,
+                              float tmin, uint32_t width_log2, uint32_t* __restrict__ prim,
+                              float* __restrict__ tout) {
+  __shared__ ChildRec root;
+  __shared__ float s_dir[3 * kHitsBlock];
+  __shared__ uint32_t s_ray[kHitsBlock];
+  __shared__ uint32_t cursor;
+  float* const dir = s_dir + threadIdx.x;
+  const uint32_t width = 1u << width_log2;
+  const uint64_t pieces = (n + width - 1) >> width_log2;
+  const uint32_t count = uint32_t((pieces - blockIdx.x + gridDim.x - 1) / gridDim.x) << width_log2;
+  if (threadIdx.x == 0) {
+    root = *s.root;
+    cursor = 0u;
+  }
+  s_ray[threadIdx.x] = kNoNode;
+  __syncthreads();
+  const unsigned lane = threadIdx.x & 31u;
+  const unsigned usable = width == 32u ? 0xffffffffu : (1u << width) - 1u;
+  const int refill = int(width * 5u / 8u);
+  auto ray_of = [&](uint32_t k) {
+    return ((uint64_t(k >> width_log2) * gridDim.x + blockIdx.x) << width_log2) + (k & (width - 1u));
+  };
+  bool exhausted = false;
+  WideRay w;
+  WideTraversal T;
+  T.cur = kNoNode;
+  uint2 st[kMaxStack];
+  for (;;) {
+    const unsigned live = __ballot_sync(0xffffffffu, T.live());
+    if (live == 0u || (!exhausted && __popc(live) <= refill)) {
+      if (!T.live() && s_ray[threadIdx.x] != kNoNode) {
+        const uint64_t i = ray_of(s_ray[threadIdx.x]);
+        const bool hit = T.rec != kNoNode;
+        prim[i] = hit ? __float_as_uint(__ldg(&s.prims[T.rec].a[3])) & ~kTagLast : 0xFFFFFFFFu;
+        tout[i] = hit ? T.closest : CUDART_INF_F;
+        s_ray[threadIdx.x] = kNoNode;
+      }
+      if (exhausted) break;
+      const unsigned idle = usable & ~live;
+      uint32_t first = 0;
+      if (lane == 0u) first = atomicAdd(&cursor, uint32_t(__popc(idle)));
+      first = __shfl_sync(0xffffffffu, first, 0);
+      exhausted = first + uint32_t(__popc(idle)) >= count;
+      const uint32_t k = first + uint32_t(__popc(idle & ((1u << lane) - 1u)));
+      if ((idle >> lane & 1u) && k < count && ray_of(k) < n) {
+        const float* r = rays + 6 * ray_of(k);
+        const RayQ q = make_ray(r[0], r[1], r[2], r[3], r[4], r[5]);
+        s_ray[threadIdx.x] = k;
+        w = make_wide_ray(q);
+        store_direction<kHitsBlock>(dir, q);
+        wide_begin(T, s.pairs, s.prims, s.root, root, q, tmin, CUDART_INF_F, false);
+      }
+    }
+    const int left = __popc(__ballot_sync(0xffffffffu, T.live()));
+    wide_round<kHitsBlock>(T, w, dir, tmin, false, s.wide, s.leaves, st, min(kNodeKeep, left >> 1));
+  }
 }
 
 __global__ void triangle_vertices_kernel(const PrimRecord* __restrict__ prims, uint32_t n,
@@ -271,8 +351,21 @@ cudaError_t launch_triangle_vertices(const PrimRecord* prims, uint32_t n, const 
 }
 
 cudaError_t launch_trace_closest(const DevScene& s, const float* rays, uint64_t n, float tmin, uint32_t* prim,
-                                 float* t, cudaStream_t stream) {
+                                 float* t, int sm_count, cudaStream_t stream) {
   if (n == 0) return cudaSuccess;
+  if (s.wide && !s.tri_verts) {
+    static const int per_sm = resident_blocks(trace_closest_wide_kernel, kHitsBlock);
+    const uint64_t blocks = uint64_t(per_sm) * sm_count, warps = blocks * (kHitsBlock / 32);
+    // Half a ray per resident warp and lane used: with 1,024 to 65,536 rays the fastest of the widths
+    // 1 to 32 was 1, 2, 8, 16 and 32 as the count grew (16,384 rays in the room: 209 us at width 1,
+    // 116 at 8, 125 at 32).
+    uint32_t width_log2 = 0;
+    while (width_log2 < 5u && (warps << width_log2) < 2 * n) ++width_log2;
+    const uint64_t block_rays = uint64_t(kHitsBlock / 32) << width_log2;
+    const uint64_t grid = std::min<uint64_t>(blocks, (n + block_rays - 1) / block_rays);
+    trace_closest_wide_kernel<<<unsigned(grid), kHitsBlock, 0, stream>>>(s, rays, n, tmin, width_log2, prim, t);
+    return cudaGetLastError();
+  }
   const int block = 128;
   const uint64_t grid = (n + block - 1) / block;
   trace_closest_kernel<<<unsigned(grid), block, 0, stream>>>(s, rays, n, tmin, prim, t);
@@ -1765,14 +1858,6 @@ __global__ void __launch_bounds__(512) wf_sort_scatter_kernel(const WavefrontLau
     const uint32_t key = i < n_ext ? W.ext_key[i] : W.shadow_key[i - n_ext];
     W.sorted[atomicAdd(&cursor[key], 1u)] = i;
   }
-}
-
-// Resident blocks per SM of a kernel at a block size.
-template <class K>
-static int resident_blocks(K kernel, int block) {
-  int blocks = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, block, 0) != cudaSuccess) return 1;
-  return blocks > 0 ? blocks : 1;
 }
 
 cudaError_t launch_wavefront_iteration(const WavefrontLaunch& w, bool moments, int sm_count, cudaStream_t stream,
