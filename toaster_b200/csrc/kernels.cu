@@ -60,6 +60,20 @@ __device__ __forceinline__ float dot(V3 a, V3 b) { return a.x * b.x + a.y * b.y 
 __device__ __forceinline__ V3 cross(V3 a, V3 b) {
   return V3{a.y * b.z - b.y * a.z, a.z * b.x - b.z * a.x, a.x * b.y - b.x * a.y};
 }
+// Dot products with every rounding written out. Left to the compiler, which product of a sum of
+// products is rounded before the fused ones depends on the kernel around it (its register cap, what
+// else is inlined), and a direction that differs in its last bit sends a path elsewhere a few bounces
+// on. So wherever the choice was seen to vary it is made here: the instantiations of the path kernel
+// (plain, with moments, guided, recording, batched) render the same paths, the wavefront's kernels
+// theirs (kWave; the two schedules always differed in these), and both stay what they were.
+__device__ __forceinline__ float dot_xyz(V3 a, V3 b) {  // x rounded, y and z fused
+  return __fmaf_rn(a.z, b.z, __fmaf_rn(a.y, b.y, __fmul_rn(a.x, b.x)));
+}
+__device__ __forceinline__ float dot_yxz(V3 a, V3 b) {  // y rounded, x and z fused
+  return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)));
+}
+template <bool kYxz>
+__device__ __forceinline__ float dot_by(V3 a, V3 b) { return kYxz ? dot_yxz(a, b) : dot_xyz(a, b); }
 __device__ __forceinline__ V3 normalize(V3 a) { return a * rsqrtf(dot(a, a)); }
 __device__ __forceinline__ V3 lerp3(V3 a, V3 b, float s) { return a + (b - a) * s; }
 
@@ -98,6 +112,22 @@ __device__ __forceinline__ float rem_euclid1(float a) {
   return r < 0.0f ? r + 1.0f : r;
 }
 
+// kCall: out of line. The path kernel, whose code does not fit the instruction cache (render_kernel),
+// keeps one copy (1.69 -> 1.65 ms with this and the texel lookup on the edit frame); the wavefront's
+// shading launch, where all warps are at the same place, inlines it (1.97 against 2.02 ms).
+__device__ __noinline__ float2 sin_cos_call(float x) {
+  float2 r;
+  sincosf(x, &r.x, &r.y);
+  return r;
+}
+template <bool kCall>
+__device__ __forceinline__ float2 sin_cos(float x) {
+  if constexpr (kCall) return sin_cos_call(x);
+  float2 r;
+  sincosf(x, &r.x, &r.y);
+  return r;
+}
+
 // environment.rs:237-241: horizontal wrap, vertical clamp.
 __device__ __forceinline__ V3 env_texel(const DevScene& s, int x, int y) {
   const int w = int(s.env_width), h = int(s.env_height);
@@ -109,8 +139,9 @@ __device__ __forceinline__ V3 env_texel(const DevScene& s, int x, int y) {
 }
 
 // environment.rs:132-152: bilinear lat-long lookup times intensity.
-__device__ V3 env_radiance(const DevScene& s, V3 d) {
-  const float l2 = dot(d, d);
+template <bool kYxz>
+__device__ __forceinline__ V3 env_radiance(const DevScene& s, V3 d) {
+  const float l2 = dot_by<kYxz>(d, d);
   if (!(l2 > 0.0f) || isinf(l2)) return mk(0.f, 0.f, 0.f);
   d = d * rsqrtf(l2);
   const float u = rem_euclid1(atan2f(d.z, d.x) / (2.0f * kPiF) + 0.5f + s.env_rotation_turns);
@@ -124,11 +155,11 @@ __device__ V3 env_radiance(const DevScene& s, V3 d) {
   const V3 bottom = lerp3(env_texel(s, x0, y0 + 1), env_texel(s, x0 + 1, y0 + 1), ax);
   return lerp3(top, bottom, ay) * s.env_intensity;
 }
-
 // environment.rs:193-200 and :225-234: density per steradian of the importance distribution.
-__device__ float env_pdf(const DevScene& s, V3 d) {
+template <bool kYxz>
+__device__ __forceinline__ float env_pdf(const DevScene& s, V3 d) {
   if (!s.env_sampleable) return 0.0f;
-  const float l2 = dot(d, d);
+  const float l2 = dot_by<kYxz>(d, d);
   if (!(l2 > 0.0f) || isinf(l2)) return 0.0f;
   d = d * rsqrtf(l2);
   const float u = rem_euclid1(atan2f(d.z, d.x) / (2.0f * kPiF) + 0.5f + s.env_rotation_turns);
@@ -147,6 +178,7 @@ __device__ float env_pdf(const DevScene& s, V3 d) {
 // columns: two dependent loads instead of a search of about twenty), with the same texel
 // probabilities. u1 draws the row, u2 the column, and the column draw's leftover fraction
 // (uniform in [0, 1) given the column) places the point across the texel; u3 places it down.
+template <bool kCall>
 __device__ bool env_sample(const DevScene& s, float u1, float u2, float u3, V3& dir, V3& rad, float& pdf) {
   if (!s.env_sampleable) return false;
   const float fy = unit_interval(u1) * float(s.env_height);
@@ -169,13 +201,12 @@ __device__ bool env_sample(const DevScene& s, float u1, float u2, float u3, V3& 
   const float v = (float(y) + unit_interval(u3)) / float(s.env_height);
   const float theta = kPiF * v;
   const float phi = 2.0f * kPiF * (u - 0.5f - s.env_rotation_turns);
-  float st, ct, sp, cp;
-  sincosf(theta, &st, &ct);
-  sincosf(phi, &sp, &cp);
+  const float2 tv = sin_cos<kCall>(theta), pv = sin_cos<kCall>(phi);
+  const float st = tv.x, ct = tv.y, sp = pv.x, cp = pv.y;
   dir = mk(st * cp, ct, st * sp);
   const float p = __ldg(s.env_pdf + size_t(y) * s.env_width + x);
   pdf = (p > 0.0f && st > 0.0f) ? p / st : 0.0f;
-  rad = env_radiance(s, dir);
+  rad = env_radiance<false>(s, dir);
   return true;
 }
 
@@ -183,11 +214,12 @@ __device__ bool env_sample(const DevScene& s, float u1, float u2, float u3, V3& 
 __device__ __forceinline__ float srgb_to_linear(float v) {
   return v <= 0.04045f ? v / 12.92f : powf((v + 0.055f) / 1.055f, 2.4f);
 }
-__device__ V3 texel_linear(const DevScene& s, const DevMaterial& m, int x, int y) {
-  const int w = int(m.tex_width), h = int(m.tex_height);
+// Out of line: a textured lookup decodes four texels of three channels, and twelve inlined powers
+// would be a sixth of every kernel that shades.
+__device__ __noinline__ V3 texel_linear(const uint32_t* texels, uint32_t offset, int w, int h, int x, int y) {
   x %= w; if (x < 0) x += w;
   y %= h; if (y < 0) y += h;
-  const uint32_t px = __ldg(s.texels + m.tex_offset + uint32_t(y) * m.tex_width + uint32_t(x));
+  const uint32_t px = __ldg(texels + offset + uint32_t(y) * uint32_t(w) + uint32_t(x));
   const float k = 1.0f / 255.0f;
   return mk(srgb_to_linear(float(px & 255u) * k), srgb_to_linear(float((px >> 8) & 255u) * k),
             srgb_to_linear(float((px >> 16) & 255u) * k));
@@ -200,21 +232,25 @@ __device__ V3 base_color(const DevScene& s, const DevMaterial& m, float tu, floa
   const float px = u * float(m.tex_width) - 0.5f, py = v * float(m.tex_height) - 0.5f;
   const int bx = int(floorf(px)), by = int(floorf(py));
   const float ax = px - floorf(px), ay = py - floorf(py);
-  const V3 top = lerp3(texel_linear(s, m, bx, by), texel_linear(s, m, bx + 1, by), ax);
-  const V3 bottom = lerp3(texel_linear(s, m, bx, by + 1), texel_linear(s, m, bx + 1, by + 1), ax);
+  const int w = int(m.tex_width), h = int(m.tex_height);
+  const V3 top = lerp3(texel_linear(s.texels, m.tex_offset, w, h, bx, by),
+                       texel_linear(s.texels, m.tex_offset, w, h, bx + 1, by), ax);
+  const V3 bottom = lerp3(texel_linear(s.texels, m.tex_offset, w, h, bx, by + 1),
+                          texel_linear(s.texels, m.tex_offset, w, h, bx + 1, by + 1), ax);
   return a * lerp3(top, bottom, ay);
 }
 
+template <bool kCall>
 __device__ __forceinline__ V3 uniform_sphere(float u1, float u2) {
   const float z = 1.0f - 2.0f * u1;
   const float r = sqrtf(fmaxf(0.0f, 1.0f - z * z));
-  float sp, cp;
-  sincosf(2.0f * kPiF * u2, &sp, &cp);
-  return mk(r * cp, r * sp, z);
+  const float2 a = sin_cos<kCall>(2.0f * kPiF * u2);
+  return mk(r * a.y, r * a.x, z);
 }
 // Uniform point in the unit ball: the distribution of random_in_unit_sphere (integrator.rs:377).
+template <bool kCall>
 __device__ __forceinline__ V3 uniform_ball(float u1, float u2, float u3) {
-  return uniform_sphere(u1, u2) * cbrtf(u3);
+  return uniform_sphere<kCall>(u1, u2) * cbrtf(u3);
 }
 __device__ __forceinline__ V3 reflect(V3 d, V3 n) { return d - 2.0f * dot(d, n) * n; }
 __device__ __forceinline__ V3 refract(V3 d, V3 n, float ratio) {
@@ -373,7 +409,8 @@ cudaError_t launch_trace_closest(const DevScene& s, const float* rays, uint64_t 
 }
 
 // ------------------------------------------------------------------------ path kernel
-enum Phase : int { kIdle = 0, kExtend = 1, kShadowLight = 2, kShadowEnv = 3, kScatter = 4 };
+// What a lane of the path kernel does next. kFinish: its sample is complete; kBegin: it starts one.
+enum Phase : int { kIdle = 0, kExtend = 1, kShadowLight = 2, kShadowEnv = 3, kScatter = 4, kFinish = 5, kBegin = 6 };
 
 // Path-id word of a training record written for an unoccluded environment shadow ray.
 constexpr uint32_t kNeeRecord = 0xFFFFFFFFu;
@@ -460,6 +497,7 @@ __device__ __forceinline__ uint32_t aggregated_increment(uint32_t* counter) {
   return base + uint32_t(__popc(active & ((1u << lane) - 1u)));
 }
 
+template <bool kWave>
 __device__ __forceinline__ void start_sample(const FrameJob& J, Lane& ln) {
   const DevScene& s = J.scene;
   ln.rng.seed(J.frame_index_dev ? *J.frame_index_dev : J.frame_index, ln.pixel, ln.sample);
@@ -481,7 +519,8 @@ __device__ __forceinline__ void start_sample(const FrameJob& J, Lane& ln) {
     vv = mk(s.cam_vertical[0], s.cam_vertical[1], s.cam_vertical[2]);
   }
   ln.ro = o;
-  ln.rd = normalize(ll + u * h + v * vv - o);
+  const V3 d = ll + u * h + v * vv - o;
+  ln.rd = d * rsqrtf(dot_by<kWave>(d, d));
   ln.thr = mk(1.f, 1.f, 1.f);
   ln.rad = mk(0.f, 0.f, 0.f);
   ln.depth = int(J.max_bounces);
@@ -515,11 +554,12 @@ __device__ __forceinline__ void finish_sample(const RenderLaunch& L, const Frame
     }
     ln.phase = kIdle;
   } else {
-    start_sample(J, ln);
+    ln.phase = kBegin;
   }
 }
 
 // Light-sampling shadow ray (integrator.rs:168-205); false when the sample contributes nothing.
+template <bool kCall>
 __device__ __forceinline__ bool prepare_light_shadow(const DevScene& s, Lane& ln) {
   if (s.light_count == 0) return false;
   const float u1 = ln.rng.uniform(), u2 = ln.rng.uniform(), u3 = ln.rng.uniform();
@@ -535,7 +575,7 @@ __device__ __forceinline__ bool prepare_light_shadow(const DevScene& s, Lane& ln
     pos = mk(lt.p0[0], lt.p0[1], lt.p0[2]) + mk(lt.e1[0], lt.e1[1], lt.e1[2]) * w1 + mk(lt.e2[0], lt.e2[1], lt.e2[2]) * w2;
     nrm = mk(lt.normal[0], lt.normal[1], lt.normal[2]);
   } else {
-    nrm = uniform_sphere(u2, u3);
+    nrm = uniform_sphere<kCall>(u2, u3);
     pos = mk(lt.p0[0], lt.p0[1], lt.p0[2]) + nrm * lt.radius;
   }
   const V3 so = ln.hp + ln.hn * kRayEps;
@@ -558,7 +598,7 @@ __device__ __forceinline__ bool prepare_light_shadow(const DevScene& s, Lane& ln
 
 // Environment-sampling shadow ray with the power heuristic (integrator.rs:208-244). At a guided
 // vertex the competing technique is the 50/50 BSDF / guide mixture, so its pdf enters the weight.
-// kWeights (and record mode): also the ray's weight as a guide training sample (ln.nee_w).
+// kWeights (the wavefront; also record mode): also the ray's weight as a guide training sample (ln.nee_w).
 template <int kMode, bool kWeights = false>
 __device__ __forceinline__ bool prepare_env_shadow(const RenderLaunch& L, const FrameJob& J, Lane& ln) {
   const DevScene& s = J.scene;
@@ -566,7 +606,7 @@ __device__ __forceinline__ bool prepare_env_shadow(const RenderLaunch& L, const 
   const float u1 = ln.rng.uniform(), u2 = ln.rng.uniform(), u3 = ln.rng.uniform();
   V3 dir, rad;
   float pdf;
-  if (!env_sample(s, u1, u2, u3, dir, rad, pdf)) return false;
+  if (!env_sample<!kWeights>(s, u1, u2, u3, dir, rad, pdf)) return false;
   const float cs = fmaxf(dot(ln.hn, dir), 0.0f);
   if (cs <= 0.0f || pdf <= 0.0f) return false;
   float indirect_pdf = cs / kPiF;
@@ -589,14 +629,15 @@ __device__ __forceinline__ bool prepare_env_shadow(const RenderLaunch& L, const 
   return true;
 }
 
+template <bool kWave>
 __device__ __forceinline__ V3 background(const DevScene& s, V3 d, float bsdf_pdf) {
   if (s.background == 0u) {
     const V3 dn = normalize(d);
     return lerp3(mk(1.f, 1.f, 1.f), mk(0.35f, 0.65f, 1.0f), 0.5f * (dn.y + 1.0f));
   }
   if (s.background != 2u || s.env_width == 0) return mk(0.f, 0.f, 0.f);
-  const V3 r = env_radiance(s, d);
-  const float w = bsdf_pdf >= 0.0f ? power_heuristic(bsdf_pdf, env_pdf(s, d)) : 1.0f;
+  const V3 r = env_radiance<kWave>(s, d);
+  const float w = bsdf_pdf >= 0.0f ? power_heuristic(bsdf_pdf, env_pdf<kWave>(s, d)) : 1.0f;
   return r * w;
 }
 
@@ -713,9 +754,10 @@ __device__ __forceinline__ Surface surface_at(const DevScene& s, V3 ro, V3 rd, c
 
 // Fuzzy metal reflection (integrator.rs:303-313): false when the ray is absorbed (it points into
 // the surface). On success the lane holds the reflected ray.
+template <bool kCall>
 __device__ __forceinline__ bool bounce_metal(Lane& ln, const DevMaterial& m, const Surface& f) {
   const V3 refl = reflect(normalize(ln.rd), f.nrm);
-  const V3 ball = uniform_ball(ln.rng.uniform(), ln.rng.uniform(), ln.rng.uniform());
+  const V3 ball = uniform_ball<kCall>(ln.rng.uniform(), ln.rng.uniform(), ln.rng.uniform());
   const V3 dir = refl + ball * m.roughness;
   if (dot(dir, f.nrm) <= 0.0f) return false;
   ln.ro = f.hp;
@@ -738,9 +780,40 @@ __device__ __forceinline__ void bounce_dielectric(Lane& ln, const DevMaterial& m
   ln.rd = normalize(dir);
 }
 
+// The same for the path kernel, with every rounding written out (see dot_xyz).
+__device__ __forceinline__ V3 scale_rn(V3 a, float k) {
+  return mk(__fmul_rn(a.x, k), __fmul_rn(a.y, k), __fmul_rn(a.z, k));
+}
+__device__ __forceinline__ V3 fma_rn(float k, V3 a, V3 b) {
+  return mk(__fmaf_rn(k, a.x, b.x), __fmaf_rn(k, a.y, b.y), __fmaf_rn(k, a.z, b.z));
+}
+__device__ __forceinline__ void bounce_dielectric_path(Lane& ln, const DevMaterial& m, const Surface& f) {
+  const float ratio = f.front ? __fdiv_rn(1.0f, m.ior) : m.ior;
+  const V3 unit = scale_rn(ln.rd, rsqrtf(dot_xyz(ln.rd, ln.rd)));
+  const float ct = fminf(dot_xyz(-unit, f.nrm), 1.0f);
+  const float st = __fsqrt_rn(__fmaf_rn(-ct, ct, 1.0f));
+  bool reflected = __fmul_rn(ratio, st) > 1.0f;
+  if (!reflected) {
+    const float q = __fdiv_rn(__fsub_rn(1.0f, ratio), __fadd_rn(1.0f, ratio));
+    const float n = __fsub_rn(1.0f, ct), n2 = __fmul_rn(n, n);
+    const float n5 = __fmul_rn(__fmul_rn(__fmul_rn(n2, n), n), n);
+    reflected = __fmaf_rn(__fmaf_rn(-q, q, 1.0f), n5, __fmul_rn(q, q)) > ln.rng.uniform();
+  }
+  V3 dir;
+  if (reflected) {
+    dir = fma_rn(__fmul_rn(-2.0f, dot_yxz(unit, f.nrm)), f.nrm, unit);
+  } else {
+    const V3 perp = scale_rn(fma_rn(ct, f.nrm, unit), ratio);
+    dir = fma_rn(-__fsqrt_rn(fabsf(__fsub_rn(1.0f, dot_yxz(perp, perp)))), f.nrm, perp);
+  }
+  ln.ro = f.hp;
+  ln.rd = scale_rn(dir, rsqrtf(dot_yxz(dir, dir)));
+}
+
 // Cosine-weighted diffuse direction about the lane's shading normal (integrator.rs:277-301).
+template <bool kCall>
 __device__ __forceinline__ V3 cosine_direction(Lane& ln) {
-  V3 dir = ln.hn + uniform_sphere(ln.rng.uniform(), ln.rng.uniform());
+  V3 dir = ln.hn + uniform_sphere<kCall>(ln.rng.uniform(), ln.rng.uniform());
   if (dot(dir, dir) < 1e-8f) dir = ln.hn;
   return normalize(dir);
 }
@@ -758,11 +831,12 @@ __device__ __forceinline__ void take_diffuse_bounce(Lane& ln, V3 dir) {
 // the mixture pdf, the guide taken with probability g.guide_fraction), so the estimator stays
 // unbiased whatever the network predicts. `mix` is the vertex's decoded mixture. False when the
 // sampled direction leaves below the surface (the path ends).
+template <bool kCall>
 __device__ __forceinline__ bool take_guided_bounce(const GuideLaunch& g, const float4* __restrict__ mix, Lane& ln) {
   const float ut = ln.rng.uniform();
   V3 dir;
   if (ut < 1.0f - g.guide_fraction) {
-    dir = cosine_direction(ln);
+    dir = cosine_direction<kCall>(ln);
   } else {
     const float a = ln.rng.uniform(), b = ln.rng.uniform(), c = ln.rng.uniform();
     dir = mix_sample(mix, a, b, c);
@@ -778,15 +852,14 @@ __device__ __forceinline__ bool take_guided_bounce(const GuideLaunch& g, const f
   return true;
 }
 
-template <int kMode, bool kMoments, bool kBatch>
-__device__ __forceinline__ void shade_hit(const RenderLaunch& L, const FrameJob& J, Lane& ln, const TraceResult& tr,
-                                          uint32_t& n_paths) {
+template <int kMode, bool kBatch>
+__device__ __forceinline__ void shade_hit(const RenderLaunch& L, const FrameJob& J, Lane& ln, const TraceResult& tr) {
   const DevScene& s = J.scene;
   const Surface f = surface_at(s, ln.ro, ln.rd, tr);
   const DevMaterial m = s.materials[f.mat];
   if (m.kind == kEmissive) {
     if (ln.include_emission) ln.rad = ln.rad + ln.thr * mk(m.emission[0], m.emission[1], m.emission[2]);
-    finish_sample<kMode, kMoments>(L, J, ln, n_paths);
+    ln.phase = kFinish;
     return;
   }
   if (m.kind == kDiffuse) {
@@ -805,12 +878,12 @@ __device__ __forceinline__ void shade_hit(const RenderLaunch& L, const FrameJob&
     return;
   }
   if (m.kind == kMetal) {
-    if (!bounce_metal(ln, m, f)) {
-      finish_sample<kMode, kMoments>(L, J, ln, n_paths);
+    if (!bounce_metal<true>(ln, m, f)) {
+      ln.phase = kFinish;
       return;
     }
   } else {
-    bounce_dielectric(ln, m, f);
+    bounce_dielectric_path(ln, m, f);
   }
   ln.include_emission = true;
   ln.bsdf_pdf = -1.0f;
@@ -821,8 +894,20 @@ __device__ __forceinline__ void shade_hit(const RenderLaunch& L, const FrameJob&
 // kPause selects the traversal: false = each ray traced to its end in one call (trace_ray);
 // true = resumable traversals that a warp pauses to refill finished lanes (dynamic ray fetching,
 // L.min_active) with an optional shared-memory short stack (L.short_stack).
+//
+// Besides traversal divergence the kernel is bound by instruction fetch: the steps of a path are most
+// of its code (94 KB), every warp is at another one, and with the end of a sample inlined at six
+// places and the steps in a loop over a switch the instruction cache missed 63 M times on a 4-spp
+// 1280x720 mixed frame (1.5 warps per issue waiting for instructions). With every step once, in order, and
+// the largest shared pieces out of line (59 KB) it misses 27 M times (0.6). At most 80 registers keep 24
+// warps per SM (guided frames, whose step after the inference is longer, run faster with 16 and no
+// spills). Kernel time, before and after: 320x180 x 4 spp of 2,051 primitives 0.65 -> 0.60 ms, mixed
+// scene 640x360 x 4 1.95 -> 1.68 and x 32 12.4 -> 10.5, an animation frame 640x360 x 16 3.92 -> 3.19, the
+// room 480x270 x 4 9.26 -> 8.84, six previews in one launch 3.65 -> 3.45, guided 320x180 x 2 2.05 -> 1.95.
+// The four-wide traversal was tried here too (with and without refills): faster in the room (5.6 ms),
+// slower on short rays (edit frame 2.0 ms, animation 4.5 ms), where its code costs fetches.
 template <int kMode, bool kMoments, bool kBatch, bool kPause>
-__global__ void __launch_bounds__(256) render_kernel(const RenderLaunch L) {
+__global__ void __launch_bounds__(256, kMode == kModeGuided && !kBatch ? 2 : 3) render_kernel(const RenderLaunch L) {
   static_assert(!kBatch || kMode != kModeRecord, "batched launches do not record training samples");
   // The root record lives in device memory (a geometry refit rewrites it between launches);
   // single-frame launches stage it in shared memory once.
@@ -858,7 +943,11 @@ __global__ void __launch_bounds__(256) render_kernel(const RenderLaunch L) {
     }
   }
 
+  // Every round runs the steps of a path once, in the order a path takes them, so each step's code is
+  // executed at most once per round, by all the lanes that are at it (the end of a sample above all:
+  // its six exits share one copy).
   for (;;) {
+    if (ln.phase == kFinish) finish_sample<kMode, kMoments>(L, frame_of<kBatch>(L, ln), ln, n_paths);
     // Refill idle lanes: one atomic per warp for all of them.
     const bool want = !finished && ln.phase == kIdle;
     const unsigned want_mask = __ballot_sync(0xffffffffu, want);
@@ -904,7 +993,7 @@ __global__ void __launch_bounds__(256) render_kernel(const RenderLaunch L) {
           ln.sample = J.sample_base + L.g.wave_first_sample + k;
           ln.acc = mk(0.f, 0.f, 0.f);
           if (kMoments) ln.acc2 = mk(0.f, 0.f, 0.f);
-          start_sample(J, ln);
+          ln.phase = kBegin;
         } else if (kMode == kModeGuided) {
           // One path per item: pixel-major within each sample of the wave.
           const uint32_t k = uint32_t(item / npix);
@@ -914,7 +1003,7 @@ __global__ void __launch_bounds__(256) render_kernel(const RenderLaunch L) {
           ln.sample = L.g.wave_first_sample + k;
           ln.acc = mk(0.f, 0.f, 0.f);
           if (kMoments) ln.acc2 = mk(0.f, 0.f, 0.f);
-          start_sample(L.f, ln);
+          ln.phase = kBegin;
         } else {
           uint64_t local = item;
           if constexpr (kBatch) {
@@ -938,53 +1027,37 @@ __global__ void __launch_bounds__(256) render_kernel(const RenderLaunch L) {
           ln.sample = J.sample_base + first;
           ln.acc = mk(0.f, 0.f, 0.f);
           if (kMoments) ln.acc2 = mk(0.f, 0.f, 0.f);
-          start_sample(J, ln);
+          ln.phase = kBegin;
         }
       }
     }
     if (__all_sync(0xffffffffu, finished)) break;
     const FrameJob& J = frame_of<kBatch>(L, ln);
     const DevScene& s = J.scene;
+    if (ln.phase == kBegin) start_sample<false>(J, ln);
 
-    // Advance the lane's state machine to its next ray.
+    // The lane's next ray: the vertex's light shadow ray, its environment shadow ray or, after the
+    // scatter (cosine-weighted diffuse bounce, integrator.rs:277-289), the extension ray.
     bool have = false;
-    while (!finished && !inflight && !have && ln.phase != kIdle) {
-      switch (ln.phase) {
-        case kExtend:
-          if (ln.depth <= 0) {
-            finish_sample<kMode, kMoments>(L, J, ln, n_paths);
-          } else {
-            have = true;
-            ln.tmax = CUDART_INF_F;
-          }
-          break;
-        case kShadowLight:
-          if (prepare_light_shadow(s, ln)) have = true;
-          else ln.phase = kShadowEnv;
-          break;
-        case kShadowEnv:
-          if (prepare_env_shadow<kMode>(L, J, ln)) have = true;
-          else ln.phase = kScatter;
-          break;
-        default: {  // kScatter: cosine-weighted diffuse bounce (integrator.rs:277-289)
-          ln.depth -= 1;
-          if (ln.depth <= 0) {
-            finish_sample<kMode, kMoments>(L, J, ln, n_paths);
-            break;
-          }
-          if constexpr (kMode == kModeGuided) {
-            if (ln.mix_slot >= 0) {
-              const float4* mix = L.g.in_mix + 10 * size_t(ln.mix_slot);
-              ln.mix_slot = -1;
-              if (!take_guided_bounce(L.g, mix, ln)) {
-                finish_sample<kMode, kMoments>(L, J, ln, n_paths);
-                break;
-              }
-              ln.phase = kExtend;
-              break;
-            }
-          }
-          const V3 dir = cosine_direction(ln);
+    if (!inflight) {
+      if (ln.phase == kShadowLight) {
+        have = prepare_light_shadow<true>(s, ln);
+        if (!have) ln.phase = kShadowEnv;
+      }
+      if (ln.phase == kShadowEnv) {
+        have = prepare_env_shadow<kMode>(L, J, ln);
+        if (!have) ln.phase = kScatter;
+      }
+      if (ln.phase == kScatter) {
+        ln.depth -= 1;
+        if (ln.depth <= 0) {
+          ln.phase = kFinish;
+        } else if (kMode == kModeGuided && ln.mix_slot >= 0) {
+          const float4* mix = L.g.in_mix + 10 * size_t(ln.mix_slot);
+          ln.mix_slot = -1;
+          ln.phase = take_guided_bounce<true>(L.g, mix, ln) ? kExtend : kFinish;
+        } else {
+          const V3 dir = cosine_direction<true>(ln);
           if constexpr (kMode == kModeRecord) {
             const uint32_t slot = aggregated_increment(L.g.record_count);
             if (slot < L.g.record_capacity) {
@@ -999,8 +1072,12 @@ __global__ void __launch_bounds__(256) render_kernel(const RenderLaunch L) {
           }
           take_diffuse_bounce(ln, dir);
           ln.phase = kExtend;
-          break;
         }
+      }
+      if (ln.phase == kExtend) {
+        have = ln.depth > 0;
+        if (have) ln.tmax = CUDART_INF_F;
+        else ln.phase = kFinish;
       }
     }
 
@@ -1070,10 +1147,10 @@ __global__ void __launch_bounds__(256) render_kernel(const RenderLaunch L) {
       } else {
         ++n_ext;
         if (!hit) {
-          ln.rad = ln.rad + ln.thr * background(s, ln.rd, ln.bsdf_pdf);
-          finish_sample<kMode, kMoments>(L, J, ln, n_paths);
+          ln.rad = ln.rad + ln.thr * background<false>(s, ln.rd, ln.bsdf_pdf);
+          ln.phase = kFinish;
         } else {
-          shade_hit<kMode, kMoments, kBatch>(L, J, ln, tr, n_paths);
+          shade_hit<kMode, kBatch>(L, J, ln, tr);
         }
       }
     }
@@ -1298,7 +1375,7 @@ __global__ void __launch_bounds__(kWfBlock) wf_logic_kernel(const WavefrontLaunc
       if (ext) {
         if (h.y == kNoNode) {
           const float4 d4 = W.ray_d[slot];
-          rad = rad + thr * background(s, mk(d4.x, d4.y, d4.z), W.ray_o[slot].w);
+          rad = rad + thr * background<true>(s, mk(d4.x, d4.y, d4.z), W.ray_o[slot].w);
           done = true;
         } else {
           const uint32_t mat = h.w & kWfMaterialMask;
@@ -1403,7 +1480,7 @@ __global__ void __launch_bounds__(kWfBlock) wf_logic_kernel(const WavefrontLaunc
         Lane ln;
         ln.pixel = uint32_t(item - uint64_t(chunk) * npix);
         ln.sample = J.sample_base + chunk;
-        start_sample(J, ln);
+        start_sample<true>(J, ln);
         W.ray_o[slot] = make_float4(ln.ro.x, ln.ro.y, ln.ro.z, -1.0f);
         W.ray_d[slot] = make_float4(ln.rd.x, ln.rd.y, ln.rd.z, 0.0f);
         W.thr[slot] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(ln.pixel));
@@ -1505,7 +1582,7 @@ __global__ void __launch_bounds__(128, 6) wf_shade_kernel(const WavefrontLaunch 
         // in the diffuse queue, in the environment NEE weight and in the bounce, as render_kernel's
         // guided mode does.
         ln.mix_slot = (kGuided && ln.depth > 1) ? int(i) : -1;
-        if (prepare_light_shadow(s, ln)) {
+        if (prepare_light_shadow<false>(s, ln)) {
           shadow_l = true;
           sl0 = make_float4(ln.ro.x, ln.ro.y, ln.ro.z, ln.tmax);
           sl1 = make_float4(ln.rd.x, ln.rd.y, ln.rd.z, __uint_as_float(2u * slot));
@@ -1527,16 +1604,16 @@ __global__ void __launch_bounds__(128, 6) wf_shade_kernel(const WavefrontLaunch 
         if (ln.depth > 0) {
           talb = ln.thr * ln.alb;
           if (kGuided && ln.mix_slot >= 0) {
-            extend = take_guided_bounce(W.r.g, W.r.g.in_mix + 10 * size_t(ln.mix_slot), ln);
+            extend = take_guided_bounce<false>(W.r.g, W.r.g.in_mix + 10 * size_t(ln.mix_slot), ln);
           } else {
-            take_diffuse_bounce(ln, cosine_direction(ln));
+            take_diffuse_bounce(ln, cosine_direction<false>(ln));
             extend = true;
           }
           bsdf_pdf = ln.bsdf_pdf;
           rec_s = extend;
         }
       } else {
-        const bool on = kind == kMetal ? bounce_metal(ln, m, f) : (bounce_dielectric(ln, m, f), true);
+        const bool on = kind == kMetal ? bounce_metal<false>(ln, m, f) : (bounce_dielectric(ln, m, f), true);
         ln.depth -= 1;
         extend = on && ln.depth > 0;
         nst |= kWfEmission;
