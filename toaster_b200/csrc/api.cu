@@ -149,7 +149,7 @@ struct tc_context {
   // Plain wavefront schedule: per-path state and queues for wf_capacity slots, and a pinned
   // ring of live-slot counts with one event per entry (the host's drain check).
   uint32_t wf_capacity = 0;
-  DevBuf wf_state, wf_ray_o, wf_ray_d, wf_thr, wf_rad, wf_rng, wf_hit, wf_nee, wf_shadow_q, wf_ext_q, wf_mat_q, wf_q;
+  DevBuf wf_state, wf_ray, wf_path, wf_rad, wf_hit, wf_nee, wf_shadow_q, wf_ext_q, wf_mat_q, wf_q;
   DevBuf wf_ext_key, wf_shadow_key, wf_sort_counts, wf_sorted;
   uint32_t* wf_live_host = nullptr;
   unsigned long long* wf_work_host = nullptr;  // the work counter, read back beside each live count
@@ -826,11 +826,9 @@ static int run_wavefront(tc_context* ctx, const tcb::RenderLaunch& L, uint32_t s
     ctx->wf_capacity = 0;
     const size_t n = cap;
     TC_CUDA(ctx, ctx->wf_state.reserve(sizeof(uint32_t) * n));
-    TC_CUDA(ctx, ctx->wf_ray_o.reserve(sizeof(float4) * n));
-    TC_CUDA(ctx, ctx->wf_ray_d.reserve(sizeof(float4) * n));
-    TC_CUDA(ctx, ctx->wf_thr.reserve(sizeof(float4) * n));
+    TC_CUDA(ctx, ctx->wf_ray.reserve(2 * sizeof(float4) * n));
+    TC_CUDA(ctx, ctx->wf_path.reserve(2 * sizeof(float4) * n));
     TC_CUDA(ctx, ctx->wf_rad.reserve(sizeof(float4) * n));
-    TC_CUDA(ctx, ctx->wf_rng.reserve(sizeof(uint4) * n));
     TC_CUDA(ctx, ctx->wf_hit.reserve(sizeof(uint4) * n));
     TC_CUDA(ctx, ctx->wf_nee.reserve(2 * sizeof(float4) * n));
     TC_CUDA(ctx, ctx->wf_shadow_q.reserve(4 * sizeof(float4) * n));  // two shadow rays per slot
@@ -850,11 +848,9 @@ static int run_wavefront(tc_context* ctx, const tcb::RenderLaunch& L, uint32_t s
   w.r = L;
   w.capacity = cap;
   w.state = ctx->wf_state.as<uint32_t>();
-  w.ray_o = ctx->wf_ray_o.as<float4>();
-  w.ray_d = ctx->wf_ray_d.as<float4>();
-  w.thr = ctx->wf_thr.as<float4>();
+  w.ray = ctx->wf_ray.as<float4>();
+  w.path = ctx->wf_path.as<float4>();
   w.rad = ctx->wf_rad.as<float4>();
-  w.rng = ctx->wf_rng.as<uint4>();
   w.hit = ctx->wf_hit.as<uint4>();
   w.nee = ctx->wf_nee.as<float4>();
   w.shadow_q = ctx->wf_shadow_q.as<float4>();

@@ -137,11 +137,11 @@ struct WavefrontLaunch {
                          // guide_fraction) and recording (records != null)
   uint32_t capacity;     // path slots
   uint32_t* state;       // state word
-  float4* ray_o;         // (ray origin.xyz, solid-angle pdf of the last diffuse bounce or -1)
-  float4* ray_d;         // (ray direction.xyz, -)
-  float4* thr;           // (throughput.xyz, pixel)
+  // Two float4 per slot side by side, one 32-byte sector: the shade and trace launches read a slot
+  // here and a slot there, and would leave half of every 16-byte array's sectors unused.
+  float4* ray;           // (origin.xyz, solid-angle pdf of the last diffuse bounce or -1), (direction.xyz, -)
+  float4* path;          // (throughput.xyz, pixel), (PCG32 state and increment)
   float4* rad;           // (radiance.xyz, the path's work item)
-  uint4* rng;            // PCG32 state and increment
   uint4* hit;            // (t bits, primitive record or kNoNode, tag, material word) of the extension ray
   float4* nee;           // 2 per slot: light and environment shadow-ray contributions
   float4* shadow_q;      // 2 per entry: (origin.xyz, tmax), (direction.xyz, target nee index)

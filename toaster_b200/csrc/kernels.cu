@@ -1319,15 +1319,24 @@ __device__ __forceinline__ void block_reserve(uint32_t* const (&counter)[N], con
     pos[i] = sh[i * kWfScanStride + kWfScanStride - 1] + sh[i * kWfScanStride + warp] + (incl[i] - n[i]);
 }
 
+__device__ __forceinline__ float4 rng_words(const Pcg& r) {
+  return make_float4(__uint_as_float(uint32_t(r.state)), __uint_as_float(uint32_t(r.state >> 32)),
+                     __uint_as_float(uint32_t(r.inc)), __uint_as_float(uint32_t(r.inc >> 32)));
+}
+
+// Bound by memory latency behind its two barriers and by the bytes of the slot state. What it loads is
+// therefore what the slot's path needs (16-spp mixed frame, sum over the frame's launches: 2.69 -> 2.59 ms
+// with the path and live counts in the reservation pass instead of two more barriers), and 32 registers
+// keep all 64 warps of an SM resident (2.59 -> 2.52; terrain 1.86 -> 1.72). Blocks of 128 / 512 / 1024:
+// 3.06 / 2.72 / 4.15 ms.
 template <bool kMoments, bool kGuided>
-__global__ void __launch_bounds__(kWfBlock) wf_logic_kernel(const WavefrontLaunch W) {
-  __shared__ uint32_t sh[4 * kWfScanStride];
+__global__ void __launch_bounds__(kWfBlock, 8) wf_logic_kernel(const WavefrontLaunch W) {
+  __shared__ uint32_t sh[5 * kWfScanStride];
   __shared__ unsigned long long s_first;
   __shared__ uint32_t s_started;
   const FrameJob& J = W.r.f;
   const DevScene& s = J.scene;
   const uint32_t npix = J.width * J.height;
-  uint32_t n_paths = 0, n_live = 0;
 
   // One slot per thread; whole warps are either in range or the last partial warp.
   {
@@ -1337,12 +1346,12 @@ __global__ void __launch_bounds__(kWfBlock) wf_logic_kernel(const WavefrontLaunc
     // Once all work is handed out, a block without a live slot starts and finishes nothing.
     if (W.work_done && !__syncthreads_or((st & kWfAlive) != 0u)) return;
     bool free_slot = valid && !(st & kWfAlive);
+    bool done = false;
     int kind = -1;
     if (st & kWfAlive) {
-      // Every load this slot may need is issued before any result is used: the state word alone
-      // decides which of them matter.
-      const float4 r4 = W.rad[slot];
-      const float4 t4 = W.thr[slot];
+      // A path's radiance is read and written only where its last vertex left shadow rays or it ends
+      // here, its throughput only where it ends: half of the slots of a mixed frame need their hit
+      // alone. The state word decides on the first loads, the hit on the rest.
       const bool nee_pending = (st & kWfNeePending) != 0u;
       const bool ext = (st & (kWfTerminate | kWfExtPending)) == kWfExtPending;
       const bool recording = W.r.g.records != nullptr;
@@ -1355,6 +1364,16 @@ __global__ void __launch_bounds__(kWfBlock) wf_logic_kernel(const WavefrontLaunc
         if (recording) rr = W.rec_ref[slot];
       }
       if (ext) h = W.hit[slot];
+      done = (st & kWfTerminate) != 0u;
+      float4 r4 = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (nee_pending || done) r4 = W.rad[slot];
+      const uint32_t hit_kind = h.w >> kWfKindShift;
+      if (ext && (h.y == kNoNode || hit_kind == uint32_t(kEmissive))) {
+        done = true;
+        if (!nee_pending) r4 = W.rad[slot];
+      }
+      float4 t4 = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (done) t4 = W.path[2 * size_t(slot)];
       V3 rad = mk(r4.x, r4.y, r4.z);
       const V3 thr = mk(t4.x, t4.y, t4.z);
       if (nee_pending) {
@@ -1371,24 +1390,17 @@ __global__ void __launch_bounds__(kWfBlock) wf_logic_kernel(const WavefrontLaunc
         }
         if (rr.y != kNoNode && nb.w == 0.0f) reinterpret_cast<float*>(W.r.g.records + 4 * size_t(rr.y) + 3)[0] = 0.0f;
       }
-      bool done = (st & kWfTerminate) != 0u;
       if (ext) {
         if (h.y == kNoNode) {
-          const float4 d4 = W.ray_d[slot];
-          rad = rad + thr * background<true>(s, mk(d4.x, d4.y, d4.z), W.ray_o[slot].w);
-          done = true;
-        } else {
-          const uint32_t mat = h.w & kWfMaterialMask;
-          const uint32_t k = h.w >> kWfKindShift;
-          if (k == kEmissive) {
-            if (st & kWfEmission) {
-              const DevMaterial& m = s.materials[mat];
-              rad = rad + thr * mk(__ldg(&m.emission[0]), __ldg(&m.emission[1]), __ldg(&m.emission[2]));
-            }
-            done = true;
-          } else {
-            kind = int(k);
+          const float4 o4 = W.ray[2 * size_t(slot)], d4 = W.ray[2 * size_t(slot) + 1];
+          rad = rad + thr * background<true>(s, mk(d4.x, d4.y, d4.z), o4.w);
+        } else if (hit_kind == uint32_t(kEmissive)) {
+          if (st & kWfEmission) {
+            const DevMaterial& m = s.materials[h.w & kWfMaterialMask];
+            rad = rad + thr * mk(__ldg(&m.emission[0]), __ldg(&m.emission[1]), __ldg(&m.emission[2]));
           }
+        } else {
+          kind = int(hit_kind);
         }
       }
       if (done) {
@@ -1405,9 +1417,8 @@ __global__ void __launch_bounds__(kWfBlock) wf_logic_kernel(const WavefrontLaunc
           atomicAdd(q2 + 2, double(r2.z));
         }
         if (recording) W.r.g.path_radiance[__float_as_uint(r4.w)] = make_float4(rad.x, rad.y, rad.z, 0.0f);
-        ++n_paths;
         free_slot = true;
-      } else {
+      } else if (nee_pending) {
         W.rad[slot] = make_float4(rad.x, rad.y, rad.z, r4.w);
       }
     }
@@ -1415,19 +1426,20 @@ __global__ void __launch_bounds__(kWfBlock) wf_logic_kernel(const WavefrontLaunc
     // material queues (paths that go on; the shade launch rewrites their state), thread 3 on the
     // work counter for free slots and then on the extension queue for the camera paths that do
     // start (the block's first s_started free slots in block order: items past the frame's last
-    // one start nothing). Consecutive work items are consecutive pixels of one sample, so a warp's
+    // one start nothing); thread 4 counts the finished paths. Consecutive work items are consecutive pixels of one sample, so a warp's
     // new rays are neighbours.
     const int warp = int(threadIdx.x >> 5);
     const unsigned m_mat[3] = {__ballot_sync(0xffffffffu, kind == 0), __ballot_sync(0xffffffffu, kind == 1),
                                __ballot_sync(0xffffffffu, kind == 2)};
-    const unsigned m_free = __ballot_sync(0xffffffffu, free_slot);
+    const unsigned m_free = __ballot_sync(0xffffffffu, free_slot), m_done = __ballot_sync(0xffffffffu, done);
     if ((threadIdx.x & 31u) == 0) {
 #pragma unroll
       for (int k = 0; k < 3; ++k) sh[k * kWfScanStride + warp] = uint32_t(__popc(m_mat[k]));
       sh[3 * kWfScanStride + warp] = uint32_t(__popc(m_free));
+      sh[4 * kWfScanStride + warp] = uint32_t(__popc(m_done));
     }
     __syncthreads();
-    if (threadIdx.x < 4u) {
+    if (threadIdx.x < 5u) {
       const int k = int(threadIdx.x);
       uint32_t run = 0;
       for (int w = 0; w < int(blockDim.x >> 5); ++w) {
@@ -1438,6 +1450,11 @@ __global__ void __launch_bounds__(kWfBlock) wf_logic_kernel(const WavefrontLaunc
       uint32_t base = 0;
       if (k < 3) {
         base = run ? atomicAdd(W.q + kWfMatCount + k, run) : 0u;
+        if (run) atomicAdd(W.q + kWfLive, run);
+      } else if (k == 4) {
+        if (run) atomicAdd(W.r.counters, (unsigned long long)run);
+      } else if (W.work_done) {
+        s_started = 0u;
       } else {
         const unsigned long long first = run ? atomicAdd(W.r.work_counter, (unsigned long long)run) : 0ull;
         const uint64_t left = first < W.r.total_items ? W.r.total_items - first : 0ull;
@@ -1445,6 +1462,7 @@ __global__ void __launch_bounds__(kWfBlock) wf_logic_kernel(const WavefrontLaunc
         s_first = first;
         s_started = n;
         base = n ? atomicAdd(W.q + kWfExtCount, n) : 0u;
+        if (n) atomicAdd(W.q + kWfLive, n);
       }
       sh[k * kWfScanStride + kWfScanStride - 1] = base;
     }
@@ -1460,7 +1478,7 @@ __global__ void __launch_bounds__(kWfBlock) wf_logic_kernel(const WavefrontLaunc
           // queue: the surface point and shading normal the shade launch will scatter from.
           // Vertices that only do next-event estimation (depth 1) get a query too, unused.
           const uint4 h = W.hit[slot];
-          const float4 o4 = W.ray_o[slot], d4 = W.ray_d[slot];
+          const float4 o4 = W.ray[2 * size_t(slot)], d4 = W.ray[2 * size_t(slot) + 1];
           TraceResult tr;
           tr.t = __uint_as_float(h.x);
           tr.rec = h.y;
@@ -1471,7 +1489,6 @@ __global__ void __launch_bounds__(kWfBlock) wf_logic_kernel(const WavefrontLaunc
         }
       }
     }
-    bool started = false;
     if (free_slot) {
       const uint32_t rank = sh[3 * kWfScanStride + warp] + uint32_t(__popc(m_free & lanes_below()));
       if (rank < s_started) {
@@ -1481,46 +1498,27 @@ __global__ void __launch_bounds__(kWfBlock) wf_logic_kernel(const WavefrontLaunc
         ln.pixel = uint32_t(item - uint64_t(chunk) * npix);
         ln.sample = J.sample_base + chunk;
         start_sample<true>(J, ln);
-        W.ray_o[slot] = make_float4(ln.ro.x, ln.ro.y, ln.ro.z, -1.0f);
-        W.ray_d[slot] = make_float4(ln.rd.x, ln.rd.y, ln.rd.z, 0.0f);
-        W.thr[slot] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(ln.pixel));
+        W.ray[2 * size_t(slot)] = make_float4(ln.ro.x, ln.ro.y, ln.ro.z, -1.0f);
+        W.ray[2 * size_t(slot) + 1] = make_float4(ln.rd.x, ln.rd.y, ln.rd.z, 0.0f);
+        W.path[2 * size_t(slot)] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(ln.pixel));
         W.rad[slot] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(uint32_t(item)));
-        W.rng[slot] = make_uint4(uint32_t(ln.rng.state), uint32_t(ln.rng.state >> 32), uint32_t(ln.rng.inc),
-                                 uint32_t(ln.rng.inc >> 32));
+        W.path[2 * size_t(slot) + 1] = rng_words(ln.rng);
         W.state[slot] = kWfAlive | kWfExtPending | kWfEmission | (uint32_t(ln.depth) & kWfDepthMask);
         const uint32_t pos = sh[3 * kWfScanStride + kWfScanStride - 1] + rank;
         W.ext_q[pos] = slot;
         if (W.sorted) W.ext_key[pos] = wf_sort_key(W, mk(0.f, 0.f, 0.f), kNoNode, false);
-        started = true;
       } else if (st & kWfAlive) {
         W.state[slot] = 0u;
       }
     }
-    n_live += (kind >= 0 || started) ? 1u : 0u;
-  }
-  // Path and live-slot counts: one atomic per block each.
-  __shared__ unsigned long long s_paths;
-  __shared__ uint32_t s_live;
-  if (threadIdx.x == 0) {
-    s_paths = 0ull;
-    s_live = 0u;
-  }
-  __syncthreads();
-  const unsigned long long tp = __reduce_add_sync(0xffffffffu, n_paths);
-  const uint32_t tl = __reduce_add_sync(0xffffffffu, n_live);
-  if ((threadIdx.x & 31u) == 0) {
-    if (tp) atomicAdd(&s_paths, tp);
-    if (tl) atomicAdd(&s_live, tl);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    if (s_paths) atomicAdd(W.r.counters, s_paths);
-    if (s_live) atomicAdd(W.q + kWfLive, s_live);
   }
 }
 
 // At most 80 registers (6 blocks of 128 per SM): the kernel waits on memory, so the warps it keeps
-// resident count for more than the few spilled words this costs.
+// resident count for more than the few spilled words this costs. It reads the slots of one material
+// here and there, so a slot's ray and its throughput and generator are one 32-byte sector each: as
+// four 16-byte arrays half of every sector was fetched for nothing (16-spp mixed frame 1.98 -> 1.65 ms,
+// terrain 1.53 -> 1.33, room 2.42 -> 2.31).
 template <bool kGuided>
 __global__ void __launch_bounds__(128, 6) wf_shade_kernel(const WavefrontLaunch W) {
   const FrameJob& J = W.r.f;
@@ -1557,14 +1555,15 @@ __global__ void __launch_bounds__(128, 6) wf_shade_kernel(const WavefrontLaunch 
     float4 sl0, sl1, se0, se1;
     uint32_t nst = kWfAlive;
     if (valid) {
-      const float4 o4 = W.ray_o[slot], d4 = W.ray_d[slot], t4 = W.thr[slot];
-      const uint4 r4 = W.rng[slot], h = W.hit[slot];
+      const float4 o4 = W.ray[2 * size_t(slot)], d4 = W.ray[2 * size_t(slot) + 1];
+      const float4 t4 = W.path[2 * size_t(slot)], r4 = W.path[2 * size_t(slot) + 1];
+      const uint4 h = W.hit[slot];
       const uint32_t st = W.state[slot];
       ln.ro = mk(o4.x, o4.y, o4.z);
       ln.rd = mk(d4.x, d4.y, d4.z);
       ln.thr = mk(t4.x, t4.y, t4.z);
-      ln.rng.state = uint64_t(r4.x) | (uint64_t(r4.y) << 32);
-      ln.rng.inc = uint64_t(r4.z) | (uint64_t(r4.w) << 32);
+      ln.rng.state = uint64_t(__float_as_uint(r4.x)) | (uint64_t(__float_as_uint(r4.y)) << 32);
+      ln.rng.inc = uint64_t(__float_as_uint(r4.z)) | (uint64_t(__float_as_uint(r4.w)) << 32);
       ln.depth = int(st & kWfDepthMask);
       TraceResult tr;
       tr.t = __uint_as_float(h.x);
@@ -1620,11 +1619,10 @@ __global__ void __launch_bounds__(128, 6) wf_shade_kernel(const WavefrontLaunch 
       }
       if (extend) nst |= kWfExtPending | (uint32_t(ln.depth) & kWfDepthMask);
       else nst |= kWfTerminate;
-      W.ray_o[slot] = make_float4(ln.ro.x, ln.ro.y, ln.ro.z, bsdf_pdf);
-      W.ray_d[slot] = make_float4(ln.rd.x, ln.rd.y, ln.rd.z, 0.0f);
-      W.thr[slot] = make_float4(ln.thr.x, ln.thr.y, ln.thr.z, t4.w);
-      W.rng[slot] = make_uint4(uint32_t(ln.rng.state), uint32_t(ln.rng.state >> 32), uint32_t(ln.rng.inc),
-                               uint32_t(ln.rng.inc >> 32));
+      W.ray[2 * size_t(slot)] = make_float4(ln.ro.x, ln.ro.y, ln.ro.z, bsdf_pdf);
+      W.ray[2 * size_t(slot) + 1] = make_float4(ln.rd.x, ln.rd.y, ln.rd.z, 0.0f);
+      W.path[2 * size_t(slot)] = make_float4(ln.thr.x, ln.thr.y, ln.thr.z, t4.w);
+      W.path[2 * size_t(slot) + 1] = rng_words(ln.rng);
       W.state[slot] = nst;
     }
     // Queue positions for this step's shadow rays, extension rays and (recording) training records:
@@ -1691,7 +1689,7 @@ __device__ __forceinline__ RayQ wf_entry_ray(const WavefrontLaunch& W, uint32_t 
   if constexpr (kSorted) i = W.sorted[i];  // sorted position -> queue entry (extension entries sort first)
   if (i < n_ext) {
     target = W.ext_q[i];
-    const float4 o = W.ray_o[target], d = W.ray_d[target];
+    const float4 o = W.ray[2 * size_t(target)], d = W.ray[2 * size_t(target) + 1];
     tmax = CUDART_INF_F;
     return make_ray(o.x, o.y, o.z, d.x, d.y, d.z);
   }
