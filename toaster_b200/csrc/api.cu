@@ -2002,15 +2002,13 @@ int tc_guide_loss_grad(tc_context* ctx, const float* samples, size_t n, float* g
   if (!ctx->has_guide) return fail(ctx, TC_ERR_STATE, "guiding parameters were never set");
   if (n == 0 || !samples) return fail(ctx, TC_ERR_INVALID, "no samples");
   TC_CUDA(ctx, cudaSetDevice(ctx->device));
-  std::vector<float> packed;
-  pack_samples(samples, n, packed);
   cudaStream_t st = ctx->stream;
-  TC_CUDA(ctx, ctx->g_in.reserve(sizeof(float) * packed.size()));
-  TC_CUDA(ctx, cudaMemcpyAsync(ctx->g_in.ptr, packed.data(), sizeof(float) * packed.size(), cudaMemcpyHostToDevice, st));
+  TC_CUDA(ctx, ctx->g_in.reserve(sizeof(float) * 10 * n));
+  TC_CUDA(ctx, cudaMemcpyAsync(ctx->g_in.ptr, samples, sizeof(float) * 10 * n, cudaMemcpyHostToDevice, st));
   TC_CUDA(ctx, cudaMemsetAsync(ctx->guide.grad, 0, sizeof(float) * (tcb::kGuideParams + 1), st));
   TC_CUDA(ctx, cudaEventRecord(ctx->ev_kernel0, st));
-  TC_CUDA(ctx, tcb::guide_launch_loss_grad(ctx->guide, ctx->g_in.as<float4>(), uint32_t(n), 1.0f / float(n),
-                                           ctx->sm_count, st));
+  TC_CUDA(ctx, tcb::guide_launch_loss_grad(ctx->guide, nullptr, uint32_t(n), 1.0f / float(n), ctx->sm_count, st, 1.0f,
+                                           3.0e38f, 0, 0, ctx->g_in.as<float>()));
   TC_CUDA(ctx, cudaEventRecord(ctx->ev_kernel1, st));
   std::vector<float> g(tcb::kGuideParams + 1);
   TC_CUDA(ctx, cudaMemcpyAsync(g.data(), ctx->guide.grad, sizeof(float) * g.size(), cudaMemcpyDeviceToHost, st));

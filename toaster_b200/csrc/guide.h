@@ -63,7 +63,8 @@ cudaError_t guide_launch_infer(const GuideDevice& g, const float4* queries, uint
 // samples of the batch are drawn (hashed indices) from the first n_total samples.
 cudaError_t guide_launch_loss_grad(const GuideDevice& g, const float4* samples, uint32_t n, float inv_batch,
                                    int sm_count, cudaStream_t stream, float w_scale = 1.0f,
-                                   float w_clamp = 3.0e38f, uint32_t gather_seed = 0, uint32_t n_total = 0);
+                                   float w_clamp = 3.0e38f, uint32_t gather_seed = 0, uint32_t n_total = 0,
+                                   const float* rows = nullptr);
 cudaError_t guide_launch_adam(GuideDevice& g, float lr, cudaStream_t stream);
 
 }  // namespace tcb
