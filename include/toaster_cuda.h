@@ -236,7 +236,7 @@ int tc_upload_scene(tc_context* ctx, const tc_scene_data* scene);
 int tc_set_triangle_test(tc_context* ctx, int test);
 
 /* Where tc_upload_scene builds the median-split hierarchy when the scene brings none: 0 = on the
- * device for scenes of at least 4,096 primitives, on the host below (default); 1 = always on the
+ * device for scenes of at least 1,024 primitives, on the host below (default); 1 = always on the
  * host; 2 = always on the device. Both builds produce the reference's tree (same topology,
  * primitive order and bounds). The device build runs level by level with a segmented stable
  * sort; a node whose centroids all coincide (a degenerate leaf of the reference) makes it fall

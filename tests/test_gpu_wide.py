@@ -90,3 +90,24 @@ def test_hits_at_every_launch_shape(renderer, count):
     want_prim, want_t = oracle.Oracle(scene).trace_closest(rays)
     assert np.array_equal(prim, want_prim)
     assert np.array_equal(t.view(np.uint32)[prim != 0xFFFFFFFF], want_t.view(np.uint32)[prim != 0xFFFFFFFF])
+
+
+# Around the size from which uploads build on the device: the automatic choice, the host build and the
+# device build must hold the same hierarchy, coincident centroids (a large leaf) included.
+@pytest.mark.parametrize("triangles,spheres,coincident",
+                         [(1020, 3, False), (1021, 3, False), (1022, 3, False), (2000, 60, False), (4090, 5, False),
+                          (1100, 40, True)])
+def test_builds_agree_around_the_device_threshold(renderer, triangles, spheres, coincident):
+    scene = scene_of(triangles, spheres, 17, coincident)
+    rays = configs.parity_rays(scene, 20001, seed=3)
+    data, hits = scene_to_gpu(scene), {}
+    for mode in ("host", "device", "auto"):
+        renderer.set_hierarchy_build(mode)
+        try:
+            renderer.upload(data)
+        finally:
+            renderer.set_hierarchy_build("auto")
+        hits[mode] = renderer.trace_closest(rays)
+    for mode in ("device", "auto"):
+        assert np.array_equal(hits[mode][0], hits["host"][0])
+        assert np.array_equal(hits[mode][1].view(np.uint32), hits["host"][1].view(np.uint32))

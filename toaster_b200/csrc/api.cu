@@ -45,8 +45,11 @@ constexpr uint64_t kWavefrontMinPaths = 1ull << 20;
 // Iterations the host runs ahead of the live-slot count it waits for (kWfRing = kWfLag + 1).
 constexpr int kWfLag = 4;
 constexpr int kWfRing = kWfLag + 1;
-// Scenes with at least this many primitives build their hierarchy on the device by default.
-constexpr size_t kDeviceBuildMin = 4096;
+// Scenes with at least this many primitives build their hierarchy on the device by default. A whole
+// upload with the host / device build (the same tree either way), repeated and into a new context: 512
+// primitives 257 / 328 and 308 / 514 us, 1,024 535 / 390 and 586 / 532, 2,048 1,067 / 442 and 1,116 / 594,
+// 4,000 2,342 / 540 and 2,364 / 749.
+constexpr size_t kDeviceBuildMin = 1024;
 // Guide training samples the pool keeps across recording batches (48 bytes each: 768 MiB).
 constexpr uint32_t kGuidePoolSamples = 1u << 24;
 

@@ -18,7 +18,7 @@ drives the reference through it can switch backends:
 
 Differences by design: the display conversion runs on the device inside ``readback`` (the
 ``conversion`` timing is zero); a frame whose geometry changed is re-uploaded, which rebuilds
-the hierarchy (on the device from 4,096 primitives), or, with ``hierarchy="refit"``, refit on
+the hierarchy (on the device from 1,024 primitives), or, with ``hierarchy="refit"``, refit on
 the device; device kernel time is reported beside the host stage timings. A scene evaluator is
 any object with ``evaluate(time_seconds, loop_cycle) -> EvaluatedScene``: the reference's
 animation tracks and physics are not part of this package.
