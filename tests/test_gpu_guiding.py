@@ -72,6 +72,28 @@ def test_guide_loss_and_gradient_match_reference(renderer):
     assert np.all(g["W1"][:, 75:] == 0.0)
 
 
+# The loss and gradient are sums over samples: a call must equal the sum of calls on its 128-sample
+# tiles, with partial tiles and with one, two and three tiles per block. Weights carry the factor n that
+# the mean divides out, so every sample's output gradient is the same up to one FP32 rounding; where that
+# flips its BF16 rounding an entry moves by at most 2^-8.
+@pytest.mark.parametrize("n", [1, 127, 129, 148 * 128 + 1, 2 * 148 * 128 + 77])
+def test_guide_gradient_is_the_sum_over_tiles(renderer, n):
+    renderer.guide_set_params(gn.init_params(seed=6), BOUNDS)
+    samples = make_samples(n, 21)
+
+    def scaled(part):
+        s = part.copy()
+        s[:, 9] *= np.float32(part.shape[0])
+        return renderer.guide_loss_grad(s)
+
+    grad, loss = scaled(samples)
+    parts = [scaled(samples[i:i + 128]) for i in range(0, n, 128)]
+    ref = np.sum([g.astype(np.float64) for g, _ in parts], axis=0)
+    size = np.sum([np.abs(g.astype(np.float64)) for g, _ in parts], axis=0)
+    assert np.linalg.norm(grad - ref) <= 2.0 ** -8 * np.linalg.norm(size)
+    assert abs(loss - sum(v for _, v in parts)) <= 1e-5 * sum(abs(v) for _, v in parts)
+
+
 def test_guide_adam_step_matches_reference(renderer):
     params = gn.init_params(seed=9)
     renderer.guide_set_params(params, BOUNDS)

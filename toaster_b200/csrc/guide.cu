@@ -374,14 +374,30 @@ constexpr int kTrainSmem = kTrainDB + 224 * 4;
 constexpr uint32_t kColFwd = 0, kColDH = 64, kColDW4 = 128, kColDW3 = 192, kColDW2 = 256, kColDW1 = 320;
 
 // Bias gradient of one tile: column sums of the 128-row K-major BF16 dZ tile (the values the
-// weight-gradient MMA consumes), added to db. Thread c < k sums column c, so no atomics are needed.
-__device__ __forceinline__ void tile_column_sums(const uint8_t* tile, int k, float* db, int tid) {
-  if (tid >= k) return;
-  float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll 8
-  for (int r = 0; r < 128; ++r)
-    acc[r & 3] += __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(tile + kmajor_offset(r, tid, k)));
-  db[tid] += (acc[0] + acc[1]) + (acc[2] + acc[3]);
+// weight-gradient MMA consumes), called while that MMA runs on the tile. A thread sums a pair of columns
+// over its warp's 32 rows (K = 64) or half of them (K = 32) and keeps the sums in registers until the
+// CTA's last tile; lanes of neighbouring column groups start at neighbouring rows, so that one load
+// covers all 32 banks. One column per thread over all rows, between the epilogue and the MMA, had half
+// the warps wait for 128 dependent shared loads four times a tile (32,768 samples: 45 -> 39 us, 131,072:
+// 117 -> 93).
+__device__ __forceinline__ void tile_column_sums(const uint8_t* tile, int k, float2& sum, int tid) {
+  const int lane = tid & 31, col = 2 * (lane & (k / 2 - 1));
+  const int split = 64 / k, groups = 4 / split;  // row groups of this thread
+  const int first = 32 * (tid >> 5) + 8 * groups * (lane / (k / 2));
+  float2 acc[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
+#pragma unroll
+  for (int g = 0; g < groups; ++g) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int row = first + 8 * g + ((i + (lane >> 2)) & 7);
+      const float2 v =
+          __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(tile + kmajor_offset(row, col, k)));
+      acc[i & 1].x += v.x;
+      acc[i & 1].y += v.y;
+    }
+  }
+  sum.x += acc[0].x + acc[1].x;
+  sum.y += acc[0].y + acc[1].y;
 }
 
 // Activation-gradient epilogue: dh (64 accumulator columns) -> dz = dh * [h > 0] -> BF16 row of the
@@ -414,7 +430,7 @@ __device__ __forceinline__ void epilogue_backward(uint32_t lane_tmem, const uint
 
 // Samples are three float4 (position and weight, normal, direction: the sample pool) or, with `rows`,
 // the caller's ten floats (position, normal, direction, weight), read as they come so that the host
-// need not repack them first (a 32,768-sample tc_guide_loss_grad: 332 -> 219 us).
+// need not repack them first (a 32,768-sample tc_guide_loss_grad: 318 -> 197 us).
 __global__ void __launch_bounds__(128, 1) guide_train_kernel(const float4* __restrict__ samples,
                                                              const float* __restrict__ rows, uint32_t n,
                                                              const uint8_t* __restrict__ img,
@@ -459,6 +475,7 @@ __global__ void __launch_bounds__(128, 1) guide_train_kernel(const float4* __res
   bool ok = true;
   float loss = 0.0f;
   bool accumulate = false;
+  float2 db[4] = {};  // bias gradients of this thread's column pairs, per layer
   const uint32_t tiles = (n + 127) / 128;
 
   auto wait_mma = [&]() {
@@ -543,8 +560,6 @@ __global__ void __launch_bounds__(128, 1) guide_train_kernel(const float4* __res
         *reinterpret_cast<uint4*>(s_dz + kmajor_offset(tid, 8 * g, 32)) = o;
       }
     }
-    __syncthreads();
-    tile_column_sums(s_dz, 32, s_db + 192, tid);
     // Backward: dH3 = dY W4 and dW4 += dY^T H3.
     sync_for_mma();
     if (tid == 0) {
@@ -552,10 +567,9 @@ __global__ void __launch_bounds__(128, 1) guide_train_kernel(const float4* __res
       issue_weight_grad(tmem + kColDW4, s_dz, 32, s_h[2], 64, 64, accumulate);
       umma::commit(&mbar);
     }
+    tile_column_sums(s_dz, 32, db[3], tid);
     if (!wait_mma()) break;
     epilogue_backward(tmem + lane + kColDH, s_h[2], s_dz, tid);
-    __syncthreads();
-    tile_column_sums(s_dz, 64, s_db + 128, tid);
     // dH2 = dZ3 W3, dW3 += dZ3^T H2.
     sync_for_mma();
     if (tid == 0) {
@@ -563,10 +577,9 @@ __global__ void __launch_bounds__(128, 1) guide_train_kernel(const float4* __res
       issue_weight_grad(tmem + kColDW3, s_dz, 64, s_h[1], 64, 64, accumulate);
       umma::commit(&mbar);
     }
+    tile_column_sums(s_dz, 64, db[2], tid);
     if (!wait_mma()) break;
     epilogue_backward(tmem + lane + kColDH, s_h[1], s_dz, tid);
-    __syncthreads();
-    tile_column_sums(s_dz, 64, s_db + 64, tid);
     // dH1 = dZ2 W2, dW2 += dZ2^T H1.
     sync_for_mma();
     if (tid == 0) {
@@ -574,16 +587,16 @@ __global__ void __launch_bounds__(128, 1) guide_train_kernel(const float4* __res
       issue_weight_grad(tmem + kColDW2, s_dz, 64, s_h[0], 64, 64, accumulate);
       umma::commit(&mbar);
     }
+    tile_column_sums(s_dz, 64, db[1], tid);
     if (!wait_mma()) break;
     epilogue_backward(tmem + lane + kColDH, s_h[0], s_dz, tid);
-    __syncthreads();
-    tile_column_sums(s_dz, 64, s_db, tid);
     // dW1 += dZ1^T X.
     sync_for_mma();
     if (tid == 0) {
       issue_weight_grad(tmem + kColDW1, s_dz, 64, s_x, 80, 80, accumulate);
       umma::commit(&mbar);
     }
+    tile_column_sums(s_dz, 64, db[0], tid);
     if (!wait_mma()) break;
     accumulate = true;
   }
@@ -593,6 +606,12 @@ __global__ void __launch_bounds__(128, 1) guide_train_kernel(const float4* __res
   // length is a multiple of 16 floats) ask a quarter of the L2's atomic rate, which bounded the launch
   // (148 CTAs: 68 -> 45 us at 32,768 samples, 32 -> 26 at 128).
   if (ok && accumulate) {
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+      const int c = 64 * l + 2 * (tid & (l < 3 ? 31 : 15));
+      atomicAdd(&s_db[c], db[l].x);
+      atomicAdd(&s_db[c + 1], db[l].y);
+    }
     auto flush = [&](uint32_t col, int rows, int cols, int off) {
       if (warp * 32 >= rows) return;
       const int r = warp * 32 + (tid & 31);
