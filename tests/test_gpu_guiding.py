@@ -46,6 +46,18 @@ def test_guide_inference_matches_reference(renderer):
     assert np.allclose(got[:, 32:].sum(1), 1.0, atol=1e-5)
 
 
+# A query's outputs do not depend on its place in the call: partial tiles, one tile per block and more
+# than one (592 blocks), bit for bit.
+@pytest.mark.parametrize("n", [1, 127, 129, 592 * 128 + 1, 2 * 592 * 128 + 77])
+def test_guide_inference_is_the_same_at_every_place(renderer, n):
+    renderer.guide_set_params(gn.init_params(seed=4), BOUNDS)
+    p, nrm = random_queries(n, 12)
+    whole = renderer.guide_infer(p, nrm)
+    parts = np.concatenate([renderer.guide_infer(p[i:i + 9999], nrm[i:i + 9999]) for i in range(0, n, 9999)])
+    assert np.all(np.isfinite(whole))
+    assert np.array_equal(whole.view(np.uint32), parts.view(np.uint32))
+
+
 def make_samples(n, seed):
     rng = np.random.default_rng(seed)
     p, nrm = random_queries(n, seed)

@@ -116,6 +116,17 @@ __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32
       : "memory");
 }
 
+// Shared -> global bulk copy (16-byte aligned, bytes a multiple of 16), after fence_async_smem and a
+// barrier; bulk_wait_read by the issuing thread before the source is written again or the CTA exits.
+__device__ __forceinline__ void bulk_copy_s2g(void* dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_addr(src)),
+               "r"(bytes)
+               : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+
 // Offset of element (r, k) in the canonical K-major layout with LBO = 128 B (K groups adjacent)
 // and SBO = (k_extent / 8) * 128 B.
 __host__ __device__ constexpr uint32_t kmajor_offset(uint32_t r, uint32_t k, uint32_t k_extent) {
