@@ -345,7 +345,7 @@ def run_ours(args):
                         "issue": None if tpi is None else {
                             "threads_per_instruction": tpi, "of": 32, "frac": tpi / 32.0,
                             "source": prof.get("source")},
-                        "kernel": "wf_trace_kernel<0, 0, 0> (wavefront trace launches)",
+                        "kernel": "wf_trace_wide_kernel (wavefront trace launches)",
                         "launches_per_step": iterations, "bytes_per_ray": bpr,
                         "algorithmic_bytes_per_launch": bpr * mean_rays / iterations,
                         "launch_ms": trace_ms / iterations,

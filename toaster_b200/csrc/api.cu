@@ -48,7 +48,7 @@ constexpr int kWfRing = kWfLag + 1;
 // Scenes with at least this many primitives build their hierarchy on the device by default. A whole
 // upload with the host / device build (the same tree either way), repeated and into a new context: 512
 // primitives 257 / 328 and 308 / 514 us, 1,024 535 / 390 and 586 / 532, 2,048 1,067 / 442 and 1,116 / 594,
-// 4,000 2,342 / 540 and 2,364 / 749.
+// 4,000 2,342 / 540 and 2,364 / 749. (A process's first device build also loads its kernels, about 5 ms.)
 constexpr size_t kDeviceBuildMin = 1024;
 // Guide training samples the pool keeps across recording batches (48 bytes each: 768 MiB).
 constexpr uint32_t kGuidePoolSamples = 1u << 24;
@@ -344,14 +344,22 @@ int check_render_params(tc_context* ctx, const tc_gpu_render_params* p) {
 
 // Sizes the buffers of the four-wide form of a hierarchy of `pairs` interior nodes over `prims`
 // primitives. Leaves the scene without one (scene.wide null: the pair traversal) when a node index
-// would not fit the traversal's 32-bit byte offsets or its stack.
+// would not fit the traversal's 32-bit byte offsets or its stack, or when it does not fit in memory.
 int reserve_wide(tc_context* ctx, size_t prims, size_t pairs, uint32_t depth) {
   ctx->scene.wide = nullptr;
   ctx->scene.leaves = nullptr;
   if (pairs > tcb::kMaxWideNodes || depth > tcb::kMaxWideDepth || prims == 0) return TC_OK;
-  TC_CUDA(ctx, ctx->wide_nodes.reserve(sizeof(tcb::WideNode) * std::max<size_t>(pairs, 1)));
-  TC_CUDA(ctx, ctx->wide_leaves.reserve(sizeof(tcb::LeafPair) * tcb::max_leaf_pairs(prims, pairs)));
-  TC_CUDA(ctx, ctx->wide_scan.reserve(sizeof(uint32_t) * tcb::wide_scan_words(prims)));
+  cudaError_t e = ctx->wide_nodes.reserve(sizeof(tcb::WideNode) * std::max<size_t>(pairs, 1));
+  if (e == cudaSuccess) e = ctx->wide_leaves.reserve(sizeof(tcb::LeafPair) * tcb::max_leaf_pairs(prims, pairs));
+  if (e == cudaSuccess) e = ctx->wide_scan.reserve(sizeof(uint32_t) * tcb::wide_scan_words(prims));
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();  // not an error of the calls that follow
+    ctx->wide_nodes.release();
+    ctx->wide_leaves.release();
+    ctx->wide_scan.release();
+    return TC_OK;
+  }
+  TC_CUDA(ctx, e);
   ctx->scene.wide = ctx->wide_nodes.as<tcb::WideNode>();
   ctx->scene.leaves = ctx->wide_leaves.as<tcb::LeafPair>();
   return TC_OK;

@@ -114,8 +114,8 @@ struct RenderLaunch {
 //           camera paths in free slots (their rays join the extension queue);
 //   shade   per material queue (diffuse, then metal, then dielectric, so a warp shades one
 //           material): next-event shadow rays and the scattered extension ray;
-//   trace   extension rays (closest hit) then shadow rays (first hit), 32 rays of one kind per
-//           warp; a shadow ray that hits something zeroes its contribution.
+//   trace   extension rays (closest hit) then shadow rays (first hit), each warp refilling its
+//           finished lanes from the queue; a shadow ray that hits something zeroes its contribution.
 // State word per slot: bits 0-23 remaining depth, then the flags below.
 constexpr uint32_t kWfDepthMask = 0x00FFFFFFu;
 constexpr uint32_t kWfAlive = 1u << 24;          // the slot holds a path
