@@ -12,6 +12,7 @@
 #include <cstring>
 #include <string>
 #include <array>
+#include <utility>
 #include <vector>
 
 #include "../../include/toaster_cuda.h"
@@ -76,6 +77,10 @@ struct DevBuf {
     if (e == cudaSuccess) bytes = n;
     else ptr = nullptr;
     return e;
+  }
+  void swap(DevBuf& o) {
+    std::swap(ptr, o.ptr);
+    std::swap(bytes, o.bytes);
   }
   template <class T>
   T* as() const { return static_cast<T*>(ptr); }
@@ -928,6 +933,21 @@ static int run_wavefront(tc_context* ctx, const tcb::RenderLaunch& L, uint32_t s
   return TC_OK;
 }
 
+// What a render's options may hold, whatever the schedule it then runs on.
+static int check_render_options(tc_context* ctx, const tc_render_options& o) {
+  const int block = o.block_size ? int(o.block_size) : 128;
+  if (block % 32 != 0 || block < 32 || block > 256)
+    return fail(ctx, TC_ERR_INVALID, "block_size must be a multiple of 32 in [32, 256]");
+  if (o.guide_record > 2)
+    return fail(ctx, TC_ERR_INVALID, "guide_record must be 0, 1 (start a new sample pool) or 2 (add to the pool)");
+  if (o.guiding && !ctx->has_guide) return fail(ctx, TC_ERR_STATE, "guided rendering needs tc_guide_set_params first");
+  if (!(o.guide_fraction >= 0.0f && o.guide_fraction < 1.0f))
+    return fail(ctx, TC_ERR_INVALID, "guide_fraction must be in [0, 1)");
+  if (o.short_stack > 16) return fail(ctx, TC_ERR_INVALID, "short_stack must be at most 16 entries");
+  if (o.refill_lanes > 32) return fail(ctx, TC_ERR_INVALID, "refill_lanes must be at most 32");
+  return TC_OK;
+}
+
 // Everything a render puts on `st` without synchronising the host: accumulation setup, the path
 // kernel (or the guided wavefront's rounds) and the counter readback into `counters_host`.
 // `timing` records the context's events around the kernels (left out while capturing a graph).
@@ -940,16 +960,8 @@ static int enqueue_render(tc_context* ctx, const tc_gpu_render_params* p, const 
                           unsigned long long* counters_host) {
   const bool moments = o.keep_moments != 0;
   const uint32_t npix = p->width * p->height;
+  if (int rc = check_render_options(ctx, o)) return rc;
   const int block = o.block_size ? int(o.block_size) : 128;
-  if (block % 32 != 0 || block < 32 || block > 256)
-    return fail(ctx, TC_ERR_INVALID, "block_size must be a multiple of 32 in [32, 256]");
-  if (o.guide_record > 2)
-    return fail(ctx, TC_ERR_INVALID, "guide_record must be 0, 1 (start a new sample pool) or 2 (add to the pool)");
-  if (o.guiding && !ctx->has_guide) return fail(ctx, TC_ERR_STATE, "guided rendering needs tc_guide_set_params first");
-  if (!(o.guide_fraction >= 0.0f && o.guide_fraction < 1.0f))
-    return fail(ctx, TC_ERR_INVALID, "guide_fraction must be in [0, 1)");
-  if (o.short_stack > 16) return fail(ctx, TC_ERR_INVALID, "short_stack must be at most 16 entries");
-  if (o.refill_lanes > 32) return fail(ctx, TC_ERR_INVALID, "refill_lanes must be at most 32");
   if (timing) TC_CUDA(ctx, cudaEventRecord(ctx->ev_begin, st));
   if (int rc = prepare_accumulation(ctx, p, moments, st)) return rc;
   ctx->stats.kernel_launches = 0;
@@ -1537,8 +1549,8 @@ static int animation_stage(tc_animation* a, const tc_scene_data* sd, uint32_t fr
   return TC_OK;
 }
 
-// Enqueues the device work of one frame (what the graph holds).
-static int animation_enqueue(tc_animation* a, cudaStream_t st) {
+// Enqueues the device work of one frame (what the graph holds): its geometry and hierarchy, then its image.
+static int animation_geometry(tc_animation* a, cudaStream_t st) {
   tc_context* ctx = a->ctx;
   TC_CUDA(ctx, cudaMemcpyAsync(a->d_frame.ptr, a->h_frame, 20 * sizeof(float), cudaMemcpyHostToDevice, st));
   if (a->update_lights && ctx->light_count)
@@ -1572,8 +1584,11 @@ static int animation_enqueue(tc_animation* a, cudaStream_t st) {
                                    ctx->prims.as<tcb::PrimRecord>(), ctx->bvh_prims,
                                    ctx->raw_spheres.as<tc_gpu_sphere>(), ctx->raw_triangles.as<tc_gpu_triangle>(), st));
   }
-  if (int rc = build_wide(ctx, ctx->bvh_prims, a->rebuild ? ctx->builder.pair_count() : uint32_t(ctx->pair_count), st))
-    return rc;
+  return build_wide(ctx, ctx->bvh_prims, a->rebuild ? ctx->builder.pair_count() : uint32_t(ctx->pair_count), st);
+}
+
+static int animation_render(tc_animation* a, cudaStream_t st) {
+  tc_context* ctx = a->ctx;
   const float* cam = a->d_frame.as<float>();
   const uint32_t* fi = reinterpret_cast<const uint32_t*>(cam + 16);
   if (int rc = enqueue_render(ctx, &a->params, a->options, st, false, fi, cam, a->h_counters)) return rc;
@@ -1595,6 +1610,13 @@ int tc_animation_create(tc_context* ctx, const tc_scene_data* first_frame, const
   if (options) o = *options;
   if (o.guide_record || o.keep_moments)
     return fail(ctx, TC_ERR_INVALID, "animation frames do not record training samples or keep moments");
+  if (int rc = check_render_options(ctx, o)) return rc;
+  if (o.schedule > TC_SCHEDULE_WAVEFRONT) return fail(ctx, TC_ERR_INVALID, "schedule must be 0 (auto), 1 or 2");
+  if (o.schedule == TC_SCHEDULE_WAVEFRONT)
+    return fail(ctx, TC_ERR_INVALID, "the wavefront schedule renders direct calls only, not captured frames");
+  if (ctx->scene.tri_verts)
+    return fail(ctx, TC_ERR_INVALID,
+                "the watertight triangle test is traced by tc_trace_closest and by plain wavefront renders only");
   TC_CUDA(ctx, cudaSetDevice(ctx->device));
   auto* a = new tc_animation();
   a->ctx = ctx;
@@ -1616,44 +1638,60 @@ int tc_animation_create(tc_context* ctx, const tc_scene_data* first_frame, const
   if (a->rebuild) {
     host(reinterpret_cast<void**>(&a->h_status), sizeof(uint32_t));
     if (ctx->any_attr) host(reinterpret_cast<void**>(&a->h_attr_flags), sizeof(uint32_t) * ctx->triangle_count);
-    if (e == cudaSuccess) e = ctx->builder.plan(ctx->sphere_count, ctx->triangle_count);
-    if (e == cudaSuccess)
-      e = ctx->pairs.reserve(sizeof(tcb::PairNode) * std::max<size_t>(ctx->builder.pair_count(), 1));
-    if (e == cudaSuccess) {
-      // The first frame below builds into these buffers; until then the scene has no wide form.
-      ctx->scene.pairs = ctx->pairs.as<tcb::PairNode>();
-      if (int rc = reserve_wide(ctx, ctx->bvh_prims, ctx->builder.pair_count(), ctx->builder.depth())) {
-        animation_free(a);
-        return rc;
-      }
-    }
-    if (e == cudaSuccess) e = ctx->build_status.reserve(sizeof(uint32_t));
-    if (e == cudaSuccess && a->h_attr_flags) e = ctx->attr_flags.reserve(sizeof(uint32_t) * ctx->triangle_count);
   }
   host(reinterpret_cast<void**>(&a->h_frame), 20 * sizeof(float));
   host(reinterpret_cast<void**>(&a->h_rgba), 4 * a->npix);
   host(reinterpret_cast<void**>(&a->h_counters), 4 * sizeof(unsigned long long));
-  if (e == cudaSuccess) e = a->d_frame.reserve(20 * sizeof(float));
+  if (e != cudaSuccess) {
+    animation_free(a);
+    return cuda_fail(ctx, e, "animation buffers");
+  }
+  // The frame is checked before anything of the uploaded scene changes, so that a refused creation
+  // leaves the scene as it was.
+  int rc = animation_stage(a, first_frame, params->frame_index);
+  if (rc != TC_OK) {
+    animation_free(a);
+    return rc;
+  }
+  e = a->d_frame.reserve(20 * sizeof(float));
   if (e == cudaSuccess) e = a->d_rgba.reserve(4 * a->npix);
+  DevBuf pairs;  // for a build of more pairs than the uploaded hierarchy has
+  if (a->rebuild) {
+    if (e == cudaSuccess) e = ctx->builder.plan(ctx->sphere_count, ctx->triangle_count);
+    const size_t need = sizeof(tcb::PairNode) * std::max<size_t>(ctx->builder.pair_count(), 1);
+    if (e == cudaSuccess && need > ctx->pairs.bytes) e = pairs.reserve(need);
+    if (e == cudaSuccess) e = ctx->build_status.reserve(sizeof(uint32_t));
+    if (e == cudaSuccess && a->h_attr_flags) e = ctx->attr_flags.reserve(sizeof(uint32_t) * ctx->triangle_count);
+  }
   if (e == cudaSuccess && ctx->sphere_count) e = ctx->raw_spheres.reserve(sizeof(tc_gpu_sphere) * ctx->sphere_count);
   if (e == cudaSuccess && ctx->triangle_count)
     e = ctx->raw_triangles.reserve(sizeof(tc_gpu_triangle) * ctx->triangle_count);
   if (e != cudaSuccess) {
-    if (a->rebuild) ctx->scene.wide = nullptr;
     animation_free(a);
     return cuda_fail(ctx, e, "animation buffers");
   }
   cudaStream_t st = ctx->stream;
-  // One direct run sizes every buffer the frame needs; the capture then records the same work.
-  int rc = animation_stage(a, first_frame, params->frame_index);
-  if (rc == TC_OK) rc = animation_enqueue(a, st);
+  // One direct run sizes every buffer the frame needs; the capture then records the same work. Its first
+  // part replaces the scene's hierarchy: the new buffers are the scene's from here on, and a context where
+  // that part fails (a CUDA error) has no scene any more.
+  if (a->rebuild) {
+    if (pairs.ptr) {
+      ctx->pairs.swap(pairs);
+      ctx->scene.pairs = ctx->pairs.as<tcb::PairNode>();
+    }
+    rc = reserve_wide(ctx, ctx->bvh_prims, ctx->builder.pair_count(), ctx->builder.depth());
+  }
+  if (rc == TC_OK) rc = animation_geometry(a, st);
+  if (rc != TC_OK) ctx->has_scene = false;
+  if (rc == TC_OK) rc = animation_render(a, st);
   if (rc == TC_OK && (e = cudaStreamSynchronize(st)) != cudaSuccess) rc = cuda_fail(ctx, e, "animation warm-up");
   if (rc == TC_OK) {
     ctx->raw_spheres_valid = ctx->raw_triangles_valid = true;
     if ((e = cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed)) != cudaSuccess) {
       rc = cuda_fail(ctx, e, "cudaStreamBeginCapture");
     } else {
-      rc = animation_enqueue(a, st);
+      rc = animation_geometry(a, st);
+      if (rc == TC_OK) rc = animation_render(a, st);
       cudaGraph_t g = nullptr;
       const cudaError_t e2 = cudaStreamEndCapture(st, &g);
       a->graph = g;
