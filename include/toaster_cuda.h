@@ -325,7 +325,10 @@ int tc_autotune(tc_context* ctx, const tc_gpu_render_params* params, const tc_re
  *                          refitting the first frame's tree. A refit is cheaper, but its boxes
  *                          loosen as primitives move apart; a rebuild keeps traversal cost flat.
  *                          A frame whose tree would need a degenerate leaf fails with
- *                          TC_ERR_DEVICE_STATUS. */
+ *                          TC_ERR_DEVICE_STATUS. When the scene was uploaded with a hierarchy of
+ *                          another shape (the caller's own, or one with a degenerate leaf), creation
+ *                          puts this one in its place for good: frames of animations created before
+ *                          then fail with TC_ERR_STATE. A creation that is refused changes nothing. */
 #define TC_ANIM_UPDATE_LIGHTS 1u
 #define TC_ANIM_REBUILD 2u
 typedef struct tc_animation tc_animation;

@@ -10,7 +10,7 @@ import pytest
 
 import oracle
 from test_gpu_wide import assert_same_image, scene_of
-from toaster_b200 import configs, native
+from toaster_b200 import configs, gpu_types as gt, native
 from toaster_b200.native import TcError
 from toaster_b200.renderer import Animation, GpuRenderer
 from toaster_b200.scene import scene_to_gpu
@@ -51,3 +51,58 @@ def test_refused_animation_leaves_the_scene(native_lib, loosened, why):
             Animation(r, first, rebuild=True, guiding=why == "guide")
         assert_hits(r, scene)
         assert_same_image(r)
+
+
+def own_tree(scene, leaf):
+    """The scene with a hierarchy that halves its primitives along x down to leaves of `leaf`."""
+    d = scene_to_gpu(scene)
+    c, rad = d.spheres["center_radius"][:, :3], d.spheres["center_radius"][:, 3:]
+    v = np.stack([d.triangles[k][:, :3] for k in ("v0", "v1", "v2")]) if len(d.triangles) else np.zeros((3, 0, 3), "f4")
+    pad = np.float32(1e-5)
+    lo = np.concatenate([c - rad, v.min(axis=0) - pad])
+    hi = np.concatenate([c + rad, v.max(axis=0) + pad])
+    nodes, order = [], np.argsort(lo[:, 0], kind="stable")
+    refs = np.zeros(len(order), gt.PRIMITIVE_REF)
+    refs["kind"], refs["index"] = order >= len(c), np.where(order >= len(c), order - len(c), order)
+
+    def add(a, b):
+        node = np.zeros(1, gt.BVH_NODE)
+        node["min"][0, :3], node["max"][0, :3] = lo[order[a:b]].min(axis=0), hi[order[a:b]].max(axis=0)
+        nodes.append(node)
+        if b - a <= leaf:
+            node["first_or_right"], node["primitive_count"] = a, b - a
+            return
+        add(a, (a + b) // 2)
+        node["first_or_right"] = len(nodes)
+        add((a + b) // 2, b)
+
+    add(0, len(order))
+    return scene_to_gpu(scene, bvh=(np.concatenate(nodes), refs))
+
+
+# Hierarchies of more (leaf 1) and of fewer pairs than the build that takes their place.
+@pytest.mark.parametrize("leaf", [1, 40])
+def test_update_after_a_rebuild_animation(native_lib, leaf):
+    scenes = [scene_of(300, 10, k) for k in (3, 4, 5, 6)]
+    with GpuRenderer(0) as r:
+        r.upload(own_tree(scenes[0], leaf))
+        assert_hits(r, scenes[0])
+        with Animation(r, scene_to_gpu(scenes[1]), rebuild=True) as a:
+            assert_hits(r, scenes[1])
+            assert_same_image(r)
+            a.frame(scene_to_gpu(scenes[2]), 1)
+        assert_hits(r, scenes[2])
+        r.update_geometry(scene_to_gpu(scenes[3]))
+        assert_hits(r, scenes[3])
+        assert_same_image(r)
+
+
+def test_frames_of_a_replaced_hierarchy_are_refused(native_lib):
+    first, moved = scene_of(300, 10, 3), scene_of(300, 10, 4)
+    with GpuRenderer(0) as r:
+        r.upload(own_tree(first, 1))
+        with Animation(r, scene_to_gpu(first)) as refit, Animation(r, scene_to_gpu(first), rebuild=True) as rebuild:
+            with pytest.raises(TcError, match="replaced the hierarchy"):
+                refit.frame(scene_to_gpu(moved), 1)
+            rebuild.frame(scene_to_gpu(moved), 1)
+        assert_hits(r, moved)

@@ -105,6 +105,10 @@ struct tc_context {
   uint32_t sphere_count = 0, triangle_count = 0, material_count = 0, light_count = 0, bvh_prims = 0;
   uint32_t bvh_depth = 0;
   size_t pair_count = 0;
+  // Whether the hierarchy has the one shape that builds of its primitive counts have (bvh_device.h): not a
+  // caller's, no degenerate leaf. `shape` counts the times an animation put one in place of another shape.
+  bool median_shape = false;
+  uint32_t shape = 0;
   // Four-wide form of the hierarchy (wide_build.cu), rewritten whenever the hierarchy changes.
   DevBuf wide_nodes, wide_leaves, wide_scan;
   bool any_attr = false;
@@ -587,7 +591,7 @@ int tc_upload_scene(tc_context* ctx, const tc_scene_data* sd) {
   const size_t n_prims = sd->sphere_count + sd->triangle_count;
   const bool given = sd->bvh_nodes && sd->bvh_node_count;
   const bool on_device = !given && (ctx->build_mode == 2 || (ctx->build_mode == 0 && n_prims >= kDeviceBuildMin));
-  bool built = false, unions = true;
+  bool built = false, unions = true, median_shape = !given;
   uint32_t pair_count = 0, prim_count = 0, depth = 0;
   if (on_device) {
     TC_CUDA(ctx, ctx->builder.plan(uint32_t(sd->sphere_count), uint32_t(sd->triangle_count)));
@@ -629,6 +633,9 @@ int tc_upload_scene(tc_context* ctx, const tc_scene_data* sd) {
     tcb::DeviceHierarchy dh;
     if (int rc = build_hierarchy(ctx, sd, true, dh)) return rc;
     if (given) unions = tcb::bounds_are_unions(dh);
+    if (dh.root.count > tcb::kMaxLeaf) median_shape = false;
+    for (const tcb::PairNode& p : dh.pairs)
+      if (std::max(p.child[0].count, p.child[1].count) > tcb::kMaxLeaf) median_shape = false;
     TC_CUDA(ctx, upload(ctx->pairs, dh.pairs.data(), dh.pairs.size(), st));
     TC_CUDA(ctx, upload(ctx->prims, dh.prims.data(), dh.prims.size(), st));
     TC_CUDA(ctx, upload(ctx->root_buf, &dh.root, 1, st));
@@ -736,6 +743,7 @@ int tc_upload_scene(tc_context* ctx, const tc_scene_data* sd) {
   ctx->stats.bvh_depth = depth;
   ctx->any_attr = any_attr;
   ctx->pair_count = pair_count;
+  ctx->median_shape = median_shape;
   ctx->device_built = built && on_device;
   ctx->raw_spheres_valid = ctx->device_built;
   ctx->raw_triangles_valid = ctx->device_built || ctx->scene.tri_verts != nullptr;
@@ -1489,6 +1497,7 @@ struct tc_animation {
   float exposure = 0.0f;
   bool update_lights = false;
   bool rebuild = false;                     // per-frame median-split build instead of a refit
+  uint32_t shape = 0;                       // tc_context.shape of the hierarchy the graph was captured with
   size_t npix = 0;
   tc_gpu_sphere* h_spheres = nullptr;       // pinned staging
   tc_gpu_triangle* h_triangles = nullptr;
@@ -1584,7 +1593,7 @@ static int animation_geometry(tc_animation* a, cudaStream_t st) {
                                    ctx->prims.as<tcb::PrimRecord>(), ctx->bvh_prims,
                                    ctx->raw_spheres.as<tc_gpu_sphere>(), ctx->raw_triangles.as<tc_gpu_triangle>(), st));
   }
-  return build_wide(ctx, ctx->bvh_prims, a->rebuild ? ctx->builder.pair_count() : uint32_t(ctx->pair_count), st);
+  return build_wide(ctx, ctx->bvh_prims, uint32_t(ctx->pair_count), st);
 }
 
 static int animation_render(tc_animation* a, cudaStream_t st) {
@@ -1596,6 +1605,23 @@ static int animation_render(tc_animation* a, cudaStream_t st) {
                                              a->exposure, a->d_rgba.as<uint32_t>(), st));
   TC_CUDA(ctx, cudaMemcpyAsync(a->h_rgba, a->d_rgba.ptr, 4 * a->npix, cudaMemcpyDeviceToHost, st));
   return TC_OK;
+}
+
+// Makes the shape of ctx->builder's plan the scene's: buffers, counts, refit plan and four-wide form, all to
+// be written by the build that follows. Captured frames of the shape before are refused from here on.
+static int take_median_shape(tc_context* ctx, DevBuf& pairs, DevBuf& refit_nodes, cudaStream_t st) {
+  ctx->pairs.swap(pairs);
+  ctx->scene.pairs = ctx->pairs.as<tcb::PairNode>();
+  ctx->refit_nodes.swap(refit_nodes);
+  ctx->refit_levels = ctx->builder.refit_levels();
+  ctx->pair_count = ctx->builder.pair_count();
+  ctx->bvh_depth = ctx->stats.bvh_depth = ctx->builder.depth();
+  ctx->median_shape = true;
+  ctx->shape += 1;
+  if (const size_t n = ctx->refit_levels.back())
+    TC_CUDA(ctx, cudaMemcpyAsync(ctx->refit_nodes.ptr, ctx->builder.refit_nodes(), sizeof(uint32_t) * n,
+                                 cudaMemcpyDeviceToDevice, st));
+  return reserve_wide(ctx, ctx->bvh_prims, ctx->pair_count, ctx->bvh_depth);
 }
 
 int tc_animation_create(tc_context* ctx, const tc_scene_data* first_frame, const tc_gpu_render_params* params,
@@ -1655,11 +1681,14 @@ int tc_animation_create(tc_context* ctx, const tc_scene_data* first_frame, const
   }
   e = a->d_frame.reserve(20 * sizeof(float));
   if (e == cudaSuccess) e = a->d_rgba.reserve(4 * a->npix);
-  DevBuf pairs;  // for a build of more pairs than the uploaded hierarchy has
+  DevBuf pairs, refit_nodes;  // of a hierarchy that takes the place of one of another shape
   if (a->rebuild) {
     if (e == cudaSuccess) e = ctx->builder.plan(ctx->sphere_count, ctx->triangle_count);
-    const size_t need = sizeof(tcb::PairNode) * std::max<size_t>(ctx->builder.pair_count(), 1);
-    if (e == cudaSuccess && need > ctx->pairs.bytes) e = pairs.reserve(need);
+    if (!ctx->median_shape) {
+      const size_t n = std::max<size_t>(ctx->builder.pair_count(), 1);
+      if (e == cudaSuccess) e = pairs.reserve(sizeof(tcb::PairNode) * n);
+      if (e == cudaSuccess) e = refit_nodes.reserve(sizeof(uint32_t) * n);
+    }
     if (e == cudaSuccess) e = ctx->build_status.reserve(sizeof(uint32_t));
     if (e == cudaSuccess && a->h_attr_flags) e = ctx->attr_flags.reserve(sizeof(uint32_t) * ctx->triangle_count);
   }
@@ -1672,15 +1701,9 @@ int tc_animation_create(tc_context* ctx, const tc_scene_data* first_frame, const
   }
   cudaStream_t st = ctx->stream;
   // One direct run sizes every buffer the frame needs; the capture then records the same work. Its first
-  // part replaces the scene's hierarchy: the new buffers are the scene's from here on, and a context where
-  // that part fails (a CUDA error) has no scene any more.
-  if (a->rebuild) {
-    if (pairs.ptr) {
-      ctx->pairs.swap(pairs);
-      ctx->scene.pairs = ctx->pairs.as<tcb::PairNode>();
-    }
-    rc = reserve_wide(ctx, ctx->bvh_prims, ctx->builder.pair_count(), ctx->builder.depth());
-  }
+  // part replaces the scene's hierarchy: a context where that fails (a CUDA error) has no scene any more.
+  if (a->rebuild && !ctx->median_shape) rc = take_median_shape(ctx, pairs, refit_nodes, st);
+  a->shape = ctx->shape;
   if (rc == TC_OK) rc = animation_geometry(a, st);
   if (rc != TC_OK) ctx->has_scene = false;
   if (rc == TC_OK) rc = animation_render(a, st);
@@ -1714,6 +1737,8 @@ int tc_animation_frame(tc_animation* a, const tc_scene_data* frame, uint32_t fra
   tc_context* ctx = a->ctx;
   if (!frame) return fail(ctx, TC_ERR_INVALID, "frame is null");
   if (rgba && n_bytes < 4 * a->npix) return fail(ctx, TC_ERR_INVALID, "output buffer holds fewer than 4*width*height bytes");
+  if (a->shape != ctx->shape)
+    return fail(ctx, TC_ERR_STATE, "another animation replaced the hierarchy this one was captured with");
   if (int rc = animation_stage(a, frame, frame_index)) return rc;
   TC_CUDA(ctx, cudaSetDevice(ctx->device));
   cudaStream_t st = ctx->stream;

@@ -20,7 +20,6 @@
 namespace tcb {
 namespace {
 
-constexpr uint32_t kMaxLeaf = 4;
 constexpr uint32_t kChunk = 1024;     // positions reduced by one warp
 constexpr uint32_t kNoParent = 0xFFFFFFFFu;
 

@@ -24,6 +24,8 @@
 
 namespace tcb {
 
+constexpr uint32_t kMaxLeaf = 4;  // primitives of a leaf that is not degenerate
+
 class DeviceBvhBuilder {
  public:
   DeviceBvhBuilder() = default;
