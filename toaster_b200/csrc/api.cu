@@ -110,7 +110,7 @@ struct tc_context {
   bool median_shape = false;
   uint32_t shape = 0;
   // Four-wide form of the hierarchy (wide_build.cu), rewritten whenever the hierarchy changes.
-  DevBuf wide_nodes, wide_leaves, wide_scan;
+  DevBuf wide_nodes, wide_leaves, wide_lanes;
   bool any_attr = false;
   // Geometry refit (tc_update_geometry): the root record, the scene-order geometry the prim
   // records are rewritten from, and pair-node indices grouped by depth.
@@ -360,12 +360,12 @@ int reserve_wide(tc_context* ctx, size_t prims, size_t pairs, uint32_t depth) {
   if (pairs > tcb::kMaxWideNodes || depth > tcb::kMaxWideDepth || prims == 0) return TC_OK;
   cudaError_t e = ctx->wide_nodes.reserve(sizeof(tcb::WideNode) * std::max<size_t>(pairs, 1));
   if (e == cudaSuccess) e = ctx->wide_leaves.reserve(sizeof(tcb::LeafPair) * tcb::max_leaf_pairs(prims, pairs));
-  if (e == cudaSuccess) e = ctx->wide_scan.reserve(sizeof(uint32_t) * tcb::wide_scan_words(prims));
+  if (e == cudaSuccess) e = ctx->wide_lanes.reserve(sizeof(uint32_t) * tcb::wide_scan_words(prims));
   if (e == cudaErrorMemoryAllocation) {
     cudaGetLastError();  // not an error of the calls that follow
     ctx->wide_nodes.release();
     ctx->wide_leaves.release();
-    ctx->wide_scan.release();
+    ctx->wide_lanes.release();
     return TC_OK;
   }
   TC_CUDA(ctx, e);
@@ -374,12 +374,16 @@ int reserve_wide(tc_context* ctx, size_t prims, size_t pairs, uint32_t depth) {
   return TC_OK;
 }
 
+tcb::WideForm wide_form(const tc_context* ctx) {
+  if (!ctx->scene.wide) return {};
+  return {ctx->wide_nodes.as<tcb::WideNode>(), ctx->wide_leaves.as<tcb::LeafPair>(), ctx->wide_lanes.as<uint32_t>()};
+}
+
 // Writes the four-wide form of the hierarchy now in ctx->pairs and ctx->prims (when it has one).
 int build_wide(tc_context* ctx, uint32_t prims, uint32_t pairs, cudaStream_t st) {
   if (!ctx->scene.wide) return TC_OK;
   TC_CUDA(ctx, tcb::launch_wide_build(ctx->pairs.as<tcb::PairNode>(), pairs, ctx->prims.as<tcb::PrimRecord>(), prims,
-                                      ctx->wide_scan.as<uint32_t>(), ctx->wide_nodes.as<tcb::WideNode>(),
-                                      ctx->wide_leaves.as<tcb::LeafPair>(), st));
+                                      wide_form(ctx), st));
   return TC_OK;
 }
 

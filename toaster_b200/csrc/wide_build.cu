@@ -3,9 +3,12 @@
 // nodes and leaf-ordered records whenever those change (upload, refit, per-frame rebuild), so every
 // way of building the hierarchy ends here and the launches can be captured in a graph.
 //
-// Leaf pairs are packed without gaps: leaf j starts at the sum of ceil(count / 2) over the leaves
-// before it, from a two-level scan over the records (per-chunk sums, their scan, then each leaf's
-// first record finds its place and writes its leaf).
+// Leaf pairs are packed without gaps: a leaf of c primitives takes the next ceil(c / 2). Where a
+// record goes is a running sum over the records before it, whatever the size of their leaves: a
+// record opens a pair when it starts a leaf or follows a full pair of its leaf. The scan therefore
+// runs over the maps (records placed, last pair half full) -> (the same, one record later), which
+// compose; a thread per leaf instead took 4 ms more on an upload with one leaf of 100,000
+// coincident spheres (coincident centroids are never split).
 #include <cuda_runtime.h>
 #include <math_constants.h>
 
@@ -20,160 +23,170 @@ constexpr int kPer = int(kWideChunk) / kBlock;
 __device__ __forceinline__ uint32_t tag_of(const PrimRecord* prims, uint32_t k) {
   return __float_as_uint(prims[k].a[3]);
 }
-
-// Pairs that record k adds: ceil(leaf size / 2) at a leaf's first record, else 0.
-__device__ __forceinline__ uint32_t pairs_at(const PrimRecord* prims, uint32_t k, uint32_t n) {
-  if (k >= n || (k > 0 && !(tag_of(prims, k - 1) & kTagLast))) return 0u;
-  uint32_t c = 1;
-  while (!(tag_of(prims, k + c - 1) & kTagLast) && k + c < n) ++c;
-  return (c + 1) / 2;
+__device__ __forceinline__ bool starts_leaf(const PrimRecord* prims, uint32_t k) {
+  return k == 0 || (tag_of(prims, k - 1) & kTagLast) != 0u;
 }
 
-// Exclusive sum of one value per thread over the block; `total` gets the block's sum.
-__device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t* sh, uint32_t& total) {
+// State before a record: pairs opened << 1 | whether the last one has room. A Step maps the low bit
+// to (pairs opened << 1 | low bit after), so applying it is an addition.
+struct Step {
+  uint32_t full, half;  // from a full last pair, from a half full one
+};
+__device__ __forceinline__ uint32_t apply(uint32_t state, Step s) {
+  return (state & ~1u) + ((state & 1u) ? s.half : s.full);
+}
+__device__ __forceinline__ Step compose(Step a, Step b) { return Step{apply(a.full, b), apply(a.half, b)}; }
+__device__ __forceinline__ Step identity() { return Step{0u, 1u}; }
+__device__ __forceinline__ Step step_of(const PrimRecord* prims, uint32_t k, uint32_t n) {
+  if (k >= n) return identity();
+  return starts_leaf(prims, k) ? Step{3u, 3u} : Step{3u, 0u};
+}
+
+// Composition of the steps of the threads before this one; `total` gets the whole block's.
+__device__ __forceinline__ Step block_exclusive(Step v, Step* sh, Step& total) {
   const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  uint32_t incl = v;
+  Step incl = v;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t u = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= unsigned(o)) incl += u;
+    const Step u{__shfl_up_sync(0xffffffffu, incl.full, o), __shfl_up_sync(0xffffffffu, incl.half, o)};
+    if (lane >= unsigned(o)) incl = compose(u, incl);
   }
   if (lane == 31u) sh[warp] = incl;
+  Step excl{__shfl_up_sync(0xffffffffu, incl.full, 1), __shfl_up_sync(0xffffffffu, incl.half, 1)};
+  if (lane == 0u) excl = identity();
   __syncthreads();
-  uint32_t before = 0, all = 0;
+  Step before = identity(), all = identity();
   for (unsigned w = 0; w < blockDim.x / 32; ++w) {
-    if (w < warp) before += sh[w];
-    all += sh[w];
+    if (w == warp) before = all;
+    all = compose(all, sh[w]);
   }
   __syncthreads();
   total = all;
-  return before + incl - v;
+  return compose(before, excl);
 }
 
-// Chunk sums; each thread owns kPer consecutive records.
-__global__ void __launch_bounds__(kBlock) leaf_sums_kernel(const PrimRecord* __restrict__ prims, uint32_t n,
-                                                           uint32_t* __restrict__ sums) {
-  __shared__ uint32_t sh[kBlock / 32];
+// Each chunk's step; a thread owns kPer consecutive records.
+__global__ void __launch_bounds__(kBlock) leaf_steps_kernel(const PrimRecord* __restrict__ prims, uint32_t n,
+                                                            Step* __restrict__ steps) {
+  __shared__ Step sh[kBlock / 32];
   const uint32_t k0 = blockIdx.x * kWideChunk + threadIdx.x * kPer;
-  uint32_t v = 0;
-  for (int i = 0; i < kPer; ++i) v += pairs_at(prims, k0 + i, n);
-  uint32_t total;
+  Step v = identity();
+  for (int i = 0; i < kPer; ++i) v = compose(v, step_of(prims, k0 + i, n));
+  Step total;
   block_exclusive(v, sh, total);
-  if (threadIdx.x == 0) sums[blockIdx.x] = total;
+  if (threadIdx.x == 0) steps[blockIdx.x] = total;
 }
 
-__global__ void __launch_bounds__(1024) leaf_scan_kernel(uint32_t* __restrict__ sums, uint32_t chunks) {
-  __shared__ uint32_t sh[32];
+// Chunk steps into the states the chunks start from (in `full`).
+__global__ void __launch_bounds__(1024) leaf_scan_kernel(Step* __restrict__ steps, uint32_t chunks) {
+  __shared__ Step sh[32];
   uint32_t run = 0;
   for (uint32_t base = 0; base < chunks; base += 1024) {
     const uint32_t i = base + threadIdx.x;
-    const uint32_t v = i < chunks ? sums[i] : 0u;
-    uint32_t total;
-    const uint32_t before = block_exclusive(v, sh, total);
-    if (i < chunks) sums[i] = run + before;
-    run += total;
+    const Step v = i < chunks ? steps[i] : identity();
+    Step total;
+    const Step before = block_exclusive(v, sh, total);
+    if (i < chunks) steps[i].full = apply(run, before);
+    run = apply(run, total);
   }
 }
 
-__device__ void write_leaf(const PrimRecord* __restrict__ prims, uint32_t k, uint32_t n, LeafPair* __restrict__ out) {
-  for (;;) {
-    LeafPair p{};
-    p.first = k;
-    bool last = false;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      if (last) break;
-      const PrimRecord r = prims[k];
-      const uint32_t tag = __float_as_uint(r.a[3]);
-      p.nv0x[i] = -r.a[0];
-      p.nv0y[i] = -r.a[1];
-      p.nv0z[i] = -r.a[2];
-      p.e1x[i] = r.b[0];
-      p.e1y[i] = r.b[1];
-      if (tag & kTagTriangle) {
-        p.e1z[i] = r.b[2];
-        p.e2x[i] = r.c[0];
-        p.ne2y[i] = -r.c[1];
-        p.ne2z[i] = -r.c[2];
-      } else {
-        p.flags |= i ? kPairSphere1 : kPairSphere0;
-      }
-      ++k;
-      last = (tag & kTagLast) != 0u || k >= n;
-    }
-    if (last) p.flags |= kPairLast;
-    *out++ = p;
-    if (last) return;
-  }
-}
-
-// slot[k] = first leaf pair of the leaf that starts at record k (other entries unused).
-__global__ void __launch_bounds__(kBlock) leaf_write_kernel(const PrimRecord* __restrict__ prims, uint32_t n,
-                                                            const uint32_t* __restrict__ sums,
-                                                            uint32_t* __restrict__ slot,
-                                                            LeafPair* __restrict__ leaves) {
-  __shared__ uint32_t sh[kBlock / 32];
+// lanes[k] = leaf pair of record k << 1 | its place there.
+__global__ void __launch_bounds__(kBlock) leaf_lanes_kernel(const PrimRecord* __restrict__ prims, uint32_t n,
+                                                            const Step* __restrict__ steps,
+                                                            uint32_t* __restrict__ lanes) {
+  __shared__ Step sh[kBlock / 32];
   const uint32_t k0 = blockIdx.x * kWideChunk + threadIdx.x * kPer;
-  uint32_t need[kPer], v = 0;
+  Step own[kPer], v = identity();
 #pragma unroll
   for (int i = 0; i < kPer; ++i) {
-    need[i] = pairs_at(prims, k0 + i, n);
-    v += need[i];
+    own[i] = step_of(prims, k0 + i, n);
+    v = compose(v, own[i]);
   }
-  uint32_t total;
-  uint32_t at = sums[blockIdx.x] + block_exclusive(v, sh, total);
+  Step total;
+  uint32_t state = apply(steps[blockIdx.x].full, block_exclusive(v, sh, total));
 #pragma unroll
   for (int i = 0; i < kPer; ++i) {
-    if (!need[i]) continue;
-    slot[k0 + i] = at;
-    write_leaf(prims, k0 + i, n, leaves + at);
-    at += need[i];
+    if (k0 + i >= n) break;
+    const uint32_t after = apply(state, own[i]);
+    // The pair opened last is the record's; it is the second one there unless it opened it.
+    lanes[k0 + i] = (((after >> 1) - 1u) << 1) | (after >> 1 == state >> 1 ? 1u : 0u);
+    state = after;
   }
 }
 
-// One thread per half of a wide node.
-__global__ void __launch_bounds__(kBlock) wide_nodes_kernel(const PairNode* __restrict__ pairs, uint32_t n,
-                                                            const uint32_t* __restrict__ slot,
-                                                            WideNode* __restrict__ nodes) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t p = i >> 1, half = i & 1u;
-  if (p >= n) return;
-  const ChildRec c = pairs[p].child[half];
-  ChildRec g[2];
-  if (c.link & kLeafBit) {
-    g[0] = c;
-    g[1] = ChildRec{CUDART_INF_F, CUDART_INF_F, CUDART_INF_F, kLeafBit, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, 0u};
+__device__ __forceinline__ uint32_t sphere_flag(uint32_t tag, uint32_t place) {
+  return (tag & kTagTriangle) ? 0u : (place ? kPairSphere1 : kPairSphere0);
+}
+
+// Record k into its leaf pair; a pair's first record writes the pair's words and, when it has no
+// second, that one's zeros.
+__device__ __forceinline__ void write_record(const PrimRecord* __restrict__ prims, uint32_t k, uint32_t n,
+                                             const uint32_t* __restrict__ lanes, LeafPair* __restrict__ leaves) {
+  const PrimRecord r = prims[k];
+  const uint32_t lane = lanes[k], place = lane & 1u, tag = __float_as_uint(r.a[3]);
+  LeafPair& p = leaves[lane >> 1];
+  write_lane(p, place, r);
+  if (place) return;
+  uint32_t flags = sphere_flag(tag, 0u);
+  if ((tag & kTagLast) || k + 1 >= n) {
+    flags |= kPairLast;
+    write_lane(p, 1u, PrimRecord{});
   } else {
-    g[0] = pairs[c.link].child[0];
-    g[1] = pairs[c.link].child[1];
+    const uint32_t next = tag_of(prims, k + 1);
+    flags |= sphere_flag(next, 1u) | ((next & kTagLast) ? kPairLast : 0u);
   }
+  p.first = k;
+  p.flags = flags;
+}
+
+// Half of a wide node: planes and links of what child `half` of pair p leads to.
+__device__ __forceinline__ void write_half(const PairNode* __restrict__ pairs, uint32_t p, uint32_t half,
+                                           const uint32_t* __restrict__ lanes, WideNode* __restrict__ nodes) {
+  ChildRec g[2];
+  wide_children(pairs, pairs[p].child[half], g);
+  write_planes(nodes[p], p, half, g);
+  uint2 links;
+  uint32_t* l = &links.x;
 #pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const uint32_t link = (g[k].link & kLeafBit) && g[k].count ? kLeafBit | slot[g[k].link & ~kLeafBit] : g[k].link;
-    const float f[6] = {g[k].min_x, g[k].max_x, g[k].min_y, g[k].max_y, g[k].min_z, g[k].max_z};
-    const uint32_t j = 2 * half + k;
-#pragma unroll
-    for (uint32_t q = 0; q < 6; ++q) nodes[p].quad[q ^ (p & 7u)][j] = __float_as_uint(f[q]);
-    nodes[p].quad[6u ^ (p & 7u)][j] = link;
+  for (int k = 0; k < 2; ++k)
+    l[k] = (g[k].link & kLeafBit) && g[k].count ? kLeafBit | (lanes[g[k].link & ~kLeafBit] >> 1) : g[k].link;
+  *reinterpret_cast<uint2*>(&nodes[p].quad[6u ^ (p & 7u)][2 * half]) = links;
+}
+
+// One thread per record, then one per half of a wide node.
+__global__ void __launch_bounds__(kBlock) wide_write_kernel(const PairNode* __restrict__ pairs, uint32_t pair_count,
+                                                            const PrimRecord* __restrict__ prims, uint32_t n,
+                                                            const WideForm wide) {
+  const uint64_t i = uint64_t(blockIdx.x) * kBlock + threadIdx.x;
+  if (i < n) {
+    write_record(prims, uint32_t(i), n, wide.lanes, wide.leaves);
+  } else {
+    const uint64_t h = i - n;
+    if (h < 2 * uint64_t(pair_count)) write_half(pairs, uint32_t(h >> 1), uint32_t(h & 1u), wide.lanes, wide.nodes);
   }
 }
 
 }  // namespace
 
-cudaError_t launch_wide_build(const PairNode* pairs, uint32_t pair_count, const PrimRecord* prims,
-                              uint32_t prim_count, uint32_t* scan, WideNode* nodes, LeafPair* leaves,
-                              cudaStream_t stream) {
+cudaError_t launch_wide_write(const PairNode* pairs, uint32_t pair_count, const PrimRecord* prims, uint32_t prim_count,
+                              const WideForm& wide, cudaStream_t stream) {
+  if (prim_count == 0) return cudaSuccess;
+  const uint64_t threads = uint64_t(prim_count) + 2 * uint64_t(pair_count);
+  wide_write_kernel<<<unsigned((threads + kBlock - 1) / kBlock), kBlock, 0, stream>>>(pairs, pair_count, prims,
+                                                                                      prim_count, wide);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_wide_build(const PairNode* pairs, uint32_t pair_count, const PrimRecord* prims, uint32_t prim_count,
+                              const WideForm& wide, cudaStream_t stream) {
   if (prim_count == 0) return cudaSuccess;
   const uint32_t chunks = (prim_count + kWideChunk - 1) / kWideChunk;
-  uint32_t* slot = scan;
-  uint32_t* sums = scan + prim_count;
-  leaf_sums_kernel<<<chunks, kBlock, 0, stream>>>(prims, prim_count, sums);
-  leaf_scan_kernel<<<1, 1024, 0, stream>>>(sums, chunks);
-  leaf_write_kernel<<<chunks, kBlock, 0, stream>>>(prims, prim_count, sums, slot, leaves);
-  if (pair_count)
-    wide_nodes_kernel<<<unsigned((2 * uint64_t(pair_count) + kBlock - 1) / kBlock), kBlock, 0, stream>>>(
-        pairs, pair_count, slot, nodes);
-  return cudaGetLastError();
+  Step* steps = reinterpret_cast<Step*>(wide.lanes + wide_lane_words(prim_count));
+  leaf_steps_kernel<<<chunks, kBlock, 0, stream>>>(prims, prim_count, steps);
+  leaf_scan_kernel<<<1, 1024, 0, stream>>>(steps, chunks);
+  leaf_lanes_kernel<<<chunks, kBlock, 0, stream>>>(prims, prim_count, steps, wide.lanes);
+  return launch_wide_write(pairs, pair_count, prims, prim_count, wide, stream);
 }
 
 }  // namespace tcb
