@@ -106,3 +106,17 @@ def test_frames_of_a_replaced_hierarchy_are_refused(native_lib):
                 refit.frame(scene_to_gpu(moved), 1)
             rebuild.frame(scene_to_gpu(moved), 1)
         assert_hits(r, moved)
+
+
+# Spheres and triangles change places between the frames' leaf orders when the hierarchy is rebuilt.
+@pytest.mark.parametrize("rebuild", [False, True])
+@pytest.mark.parametrize("triangles,spheres", [(0, 3), (7, 2), (700, 60)])
+def test_four_wide_form_follows_captured_frames(native_lib, triangles, spheres, rebuild):
+    scenes = [scene_of(triangles, spheres, k) for k in (7, 8, 9)]
+    with GpuRenderer(0) as r:
+        r.upload(scene_to_gpu(scenes[0]))
+        with Animation(r, scene_to_gpu(scenes[0]), rebuild=rebuild) as a:
+            for k in (1, 2):
+                a.frame(scene_to_gpu(scenes[k]), k)
+                assert_hits(r, scenes[k])
+                assert_same_image(r)

@@ -380,10 +380,12 @@ tcb::WideForm wide_form(const tc_context* ctx) {
 }
 
 // Writes the four-wide form of the hierarchy now in ctx->pairs and ctx->prims (when it has one).
-int build_wide(tc_context* ctx, uint32_t prims, uint32_t pairs, cudaStream_t st) {
+// new_shape: the form was not built before, or for a hierarchy of another shape.
+int build_wide(tc_context* ctx, uint32_t prims, uint32_t pairs, bool new_shape, cudaStream_t st) {
   if (!ctx->scene.wide) return TC_OK;
-  TC_CUDA(ctx, tcb::launch_wide_build(ctx->pairs.as<tcb::PairNode>(), pairs, ctx->prims.as<tcb::PrimRecord>(), prims,
-                                      wide_form(ctx), st));
+  const auto launch = new_shape ? tcb::launch_wide_build : tcb::launch_wide_write;
+  TC_CUDA(ctx, launch(ctx->pairs.as<tcb::PairNode>(), pairs, ctx->prims.as<tcb::PrimRecord>(), prims, wide_form(ctx),
+                      st));
   return TC_OK;
 }
 
@@ -674,9 +676,10 @@ int tc_upload_scene(tc_context* ctx, const tc_scene_data* sd) {
   s.pairs = ctx->pairs.as<tcb::PairNode>();
   s.prims = ctx->prims.as<tcb::PrimRecord>();
   s.root = ctx->root_buf.as<tcb::ChildRec>();
-  if (unions) {
+  const bool watertight = ctx->triangle_test == TC_TRIANGLE_WATERTIGHT && sd->triangle_count;
+  if (unions && !watertight) {  // the watertight test is traced through the pairs
     if (int rc = reserve_wide(ctx, prim_count, pair_count, depth)) return rc;
-    if (int rc = build_wide(ctx, prim_count, pair_count, st)) return rc;
+    if (int rc = build_wide(ctx, prim_count, pair_count, true, st)) return rc;
   }
   s.materials = ctx->materials.as<tcb::DevMaterial>();
   s.material_count = n_mat;
@@ -728,7 +731,7 @@ int tc_upload_scene(tc_context* ctx, const tc_scene_data* sd) {
     s.cam_vertical[c] = sd->camera.vertical[c];
   }
   const bool raw_tris_on_device = built && on_device;
-  if (ctx->triangle_test == TC_TRIANGLE_WATERTIGHT && sd->triangle_count) {
+  if (watertight) {
     // Vertex records for the watertight test, gathered in leaf order from the scene's triangles.
     if (!raw_tris_on_device) TC_CUDA(ctx, upload(ctx->raw_triangles, sd->triangles, sd->triangle_count, st));
     TC_CUDA(ctx, ctx->tri_verts.reserve(3 * sizeof(float4) * size_t(prim_count)));
@@ -806,8 +809,8 @@ int tc_update_geometry(tc_context* ctx, const tc_scene_data* sd, const tc_scene_
     plan.level_offsets = ctx->refit_levels;
     TC_CUDA(ctx, tcb::launch_refit(plan, ctx->pairs.as<tcb::PairNode>(), ctx->root_buf.as<tcb::ChildRec>(),
                                    ctx->prims.as<tcb::PrimRecord>(), ctx->bvh_prims,
-                                   ctx->raw_spheres.as<tc_gpu_sphere>(), ctx->raw_triangles.as<tc_gpu_triangle>(), st));
-    if (int rc = build_wide(ctx, ctx->bvh_prims, uint32_t(ctx->pair_count), st)) return rc;
+                                   ctx->raw_spheres.as<tc_gpu_sphere>(), ctx->raw_triangles.as<tc_gpu_triangle>(),
+                                   wide_form(ctx), st));
     if (ctx->scene.tri_verts && changes->triangles)
       TC_CUDA(ctx, tcb::launch_triangle_vertices(ctx->prims.as<tcb::PrimRecord>(), ctx->bvh_prims,
                                                  ctx->raw_triangles.ptr, ctx->tri_verts.as<float4>(), st));
@@ -1563,7 +1566,8 @@ static int animation_stage(tc_animation* a, const tc_scene_data* sd, uint32_t fr
 }
 
 // Enqueues the device work of one frame (what the graph holds): its geometry and hierarchy, then its image.
-static int animation_geometry(tc_animation* a, cudaStream_t st) {
+// new_shape: the scene's four-wide form was last built for a hierarchy of another shape.
+static int animation_geometry(tc_animation* a, bool new_shape, cudaStream_t st) {
   tc_context* ctx = a->ctx;
   TC_CUDA(ctx, cudaMemcpyAsync(a->d_frame.ptr, a->h_frame, 20 * sizeof(float), cudaMemcpyHostToDevice, st));
   if (a->update_lights && ctx->light_count)
@@ -1589,15 +1593,17 @@ static int animation_geometry(tc_animation* a, cudaStream_t st) {
                                     ctx->pairs.as<tcb::PairNode>(), ctx->root_buf.as<tcb::ChildRec>(),
                                     ctx->prims.as<tcb::PrimRecord>(), ctx->build_status.as<uint32_t>(), st));
     TC_CUDA(ctx, cudaMemcpyAsync(a->h_status, ctx->build_status.ptr, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    if (int rc = build_wide(ctx, ctx->bvh_prims, uint32_t(ctx->pair_count), new_shape, st)) return rc;
   } else {
     tcb::RefitPlan plan;
     plan.nodes = ctx->refit_nodes.as<uint32_t>();
     plan.level_offsets = ctx->refit_levels;
     TC_CUDA(ctx, tcb::launch_refit(plan, ctx->pairs.as<tcb::PairNode>(), ctx->root_buf.as<tcb::ChildRec>(),
                                    ctx->prims.as<tcb::PrimRecord>(), ctx->bvh_prims,
-                                   ctx->raw_spheres.as<tc_gpu_sphere>(), ctx->raw_triangles.as<tc_gpu_triangle>(), st));
+                                   ctx->raw_spheres.as<tc_gpu_sphere>(), ctx->raw_triangles.as<tc_gpu_triangle>(),
+                                   wide_form(ctx), st));
   }
-  return build_wide(ctx, ctx->bvh_prims, uint32_t(ctx->pair_count), st);
+  return TC_OK;
 }
 
 static int animation_render(tc_animation* a, cudaStream_t st) {
@@ -1706,9 +1712,10 @@ int tc_animation_create(tc_context* ctx, const tc_scene_data* first_frame, const
   cudaStream_t st = ctx->stream;
   // One direct run sizes every buffer the frame needs; the capture then records the same work. Its first
   // part replaces the scene's hierarchy: a context where that fails (a CUDA error) has no scene any more.
-  if (a->rebuild && !ctx->median_shape) rc = take_median_shape(ctx, pairs, refit_nodes, st);
+  const bool new_shape = a->rebuild && !ctx->median_shape;
+  if (new_shape) rc = take_median_shape(ctx, pairs, refit_nodes, st);
   a->shape = ctx->shape;
-  if (rc == TC_OK) rc = animation_geometry(a, st);
+  if (rc == TC_OK) rc = animation_geometry(a, new_shape, st);
   if (rc != TC_OK) ctx->has_scene = false;
   if (rc == TC_OK) rc = animation_render(a, st);
   if (rc == TC_OK && (e = cudaStreamSynchronize(st)) != cudaSuccess) rc = cuda_fail(ctx, e, "animation warm-up");
@@ -1717,7 +1724,7 @@ int tc_animation_create(tc_context* ctx, const tc_scene_data* first_frame, const
     if ((e = cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed)) != cudaSuccess) {
       rc = cuda_fail(ctx, e, "cudaStreamBeginCapture");
     } else {
-      rc = animation_geometry(a, st);
+      rc = animation_geometry(a, false, st);
       if (rc == TC_OK) rc = animation_render(a, st);
       cudaGraph_t g = nullptr;
       const cudaError_t e2 = cudaStreamEndCapture(st, &g);

@@ -9,6 +9,7 @@
 
 #include "../../include/toaster_cuda.h"
 #include "layout.h"
+#include "wide_build.h"
 
 namespace tcb {
 
@@ -20,10 +21,11 @@ struct RefitPlan {
 };
 
 // Rewrites the primitive records from the new geometry (sph / tri in scene order, device memory)
-// and recomputes every child box bottom-up, then the root record (device memory).
+// and recomputes every child box bottom-up, then the root record (device memory). `wide`: the
+// hierarchy's four-wide form, or none; the launches that hold its new values write them there too.
 cudaError_t launch_refit(const RefitPlan& plan, PairNode* pairs, ChildRec* root, PrimRecord* prims,
                          uint32_t prim_count, const tc_gpu_sphere* sph, const tc_gpu_triangle* tri,
-                         cudaStream_t stream);
+                         const WideForm& wide, cudaStream_t stream);
 
 }  // namespace tcb
 
