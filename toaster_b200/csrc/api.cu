@@ -676,11 +676,6 @@ int tc_upload_scene(tc_context* ctx, const tc_scene_data* sd) {
   s.pairs = ctx->pairs.as<tcb::PairNode>();
   s.prims = ctx->prims.as<tcb::PrimRecord>();
   s.root = ctx->root_buf.as<tcb::ChildRec>();
-  const bool watertight = ctx->triangle_test == TC_TRIANGLE_WATERTIGHT && sd->triangle_count;
-  if (unions && !watertight) {  // the watertight test is traced through the pairs
-    if (int rc = reserve_wide(ctx, prim_count, pair_count, depth)) return rc;
-    if (int rc = build_wide(ctx, prim_count, pair_count, true, st)) return rc;
-  }
   s.materials = ctx->materials.as<tcb::DevMaterial>();
   s.material_count = n_mat;
   s.lights = sd->light_count ? ctx->lights.as<tcb::DevLight>() : nullptr;
@@ -731,6 +726,7 @@ int tc_upload_scene(tc_context* ctx, const tc_scene_data* sd) {
     s.cam_vertical[c] = sd->camera.vertical[c];
   }
   const bool raw_tris_on_device = built && on_device;
+  const bool watertight = ctx->triangle_test == TC_TRIANGLE_WATERTIGHT && sd->triangle_count;
   if (watertight) {
     // Vertex records for the watertight test, gathered in leaf order from the scene's triangles.
     if (!raw_tris_on_device) TC_CUDA(ctx, upload(ctx->raw_triangles, sd->triangles, sd->triangle_count, st));
@@ -738,6 +734,12 @@ int tc_upload_scene(tc_context* ctx, const tc_scene_data* sd) {
     TC_CUDA(ctx, tcb::launch_triangle_vertices(ctx->prims.as<tcb::PrimRecord>(), prim_count, ctx->raw_triangles.ptr,
                                                ctx->tri_verts.as<float4>(), st));
     s.tri_verts = ctx->tri_verts.as<float4>();
+  }
+  // Last, out of the memory that the rest leaves: a scene can do without it. The watertight test is traced
+  // through the pairs.
+  if (unions && !watertight) {
+    if (int rc = reserve_wide(ctx, prim_count, pair_count, depth)) return rc;
+    if (int rc = build_wide(ctx, prim_count, pair_count, true, st)) return rc;
   }
   TC_CUDA(ctx, cudaStreamSynchronize(st));
   ctx->has_scene = true;
