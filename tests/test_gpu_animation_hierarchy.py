@@ -120,3 +120,16 @@ def test_four_wide_form_follows_captured_frames(native_lib, triangles, spheres, 
                 a.frame(scene_to_gpu(scenes[k]), k)
                 assert_hits(r, scenes[k])
                 assert_same_image(r)
+
+
+def test_refused_upload_leaves_the_scene(native_lib):
+    scene, other = scene_of(300, 10, 3), scene_of(900, 30, 4)
+    bad = given(other, False)
+    leaf = np.nonzero(bad.bvh_nodes["primitive_count"])[0]
+    bad.bvh_nodes["first_or_right"][leaf[3]] = bad.bvh_nodes["first_or_right"][leaf[2]]
+    with GpuRenderer(0) as r:
+        r.upload(scene_to_gpu(scene))
+        with pytest.raises(TcError, match="overlap|in no leaf"):
+            r.upload(bad)
+        assert_hits(r, scene)
+        assert_same_image(r)

@@ -599,6 +599,12 @@ int tc_upload_scene(tc_context* ctx, const tc_scene_data* sd) {
   const bool on_device = !given && (ctx->build_mode == 2 || (ctx->build_mode == 0 && n_prims >= kDeviceBuildMin));
   bool built = false, unions = true, median_shape = !given;
   uint32_t pair_count = 0, prim_count = 0, depth = 0;
+  tcb::DeviceHierarchy dh;
+  if (!on_device)
+    if (int rc = build_hierarchy(ctx, sd, true, dh)) return rc;
+  // Nothing is refused below; what can still fail are allocations and launches, between which buffers of
+  // the scene before and of this one stand side by side. A context where one fails has no scene.
+  ctx->has_scene = false;
   if (on_device) {
     TC_CUDA(ctx, ctx->builder.plan(uint32_t(sd->sphere_count), uint32_t(sd->triangle_count)));
     TC_CUDA(ctx, upload(ctx->raw_spheres, sd->spheres, sd->sphere_count, st));
@@ -636,8 +642,8 @@ int tc_upload_scene(tc_context* ctx, const tc_scene_data* sd) {
     }
   }
   if (!built) {
-    tcb::DeviceHierarchy dh;
-    if (int rc = build_hierarchy(ctx, sd, true, dh)) return rc;
+    if (on_device)
+      if (int rc = build_hierarchy(ctx, sd, true, dh)) return rc;
     if (given) unions = tcb::bounds_are_unions(dh);
     if (dh.root.count > tcb::kMaxLeaf) median_shape = false;
     for (const tcb::PairNode& p : dh.pairs)
@@ -1750,6 +1756,7 @@ int tc_animation_frame(tc_animation* a, const tc_scene_data* frame, uint32_t fra
   tc_context* ctx = a->ctx;
   if (!frame) return fail(ctx, TC_ERR_INVALID, "frame is null");
   if (rgba && n_bytes < 4 * a->npix) return fail(ctx, TC_ERR_INVALID, "output buffer holds fewer than 4*width*height bytes");
+  if (!ctx->has_scene) return fail(ctx, TC_ERR_STATE, "frame before tc_upload_scene");
   if (a->shape != ctx->shape)
     return fail(ctx, TC_ERR_STATE, "another animation replaced the hierarchy this one was captured with");
   if (int rc = animation_stage(a, frame, frame_index)) return rc;
