@@ -240,7 +240,7 @@ int tc_set_triangle_test(tc_context* ctx, int test);
  * host; 2 = always on the device. Both builds produce the reference's tree (same topology,
  * primitive order and bounds). The device build runs level by level with a segmented stable
  * sort; a node whose centroids all coincide (a degenerate leaf of the reference) makes it fall
- * back to the host build. Replaces the host-side FlatBvh::build of scene_upload.rs:296-340. */
+ * back to the host build, where below 4,096 primitives the context's next upload then starts. Replaces the host-side FlatBvh::build of scene_upload.rs:296-340. */
 int tc_set_hierarchy_build(tc_context* ctx, int mode);
 
 /* Replaces the camera write_buffer (path_tracer.rs:680-684). */

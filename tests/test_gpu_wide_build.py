@@ -45,3 +45,25 @@ def test_leaves_of_every_size(renderer, sizes):
     assert_same_image(renderer)
     renderer.update_geometry(scene_to_gpu(moved))
     assert_same_image(renderer)
+
+
+# The automatic choice of the builder remembers a degenerate leaf below 4,096 primitives: whatever came
+# before, each scene gets the hierarchy of a host build.
+def test_build_choice_after_a_degenerate_leaf(renderer):
+    regular, degenerate = scene_of(1500, 20, 2), scene_of(1500, 20, 2, coincident=True)
+    rays = configs.parity_rays(regular, 5001, seed=2)
+
+    def hits(scene, mode):
+        renderer.set_hierarchy_build(mode)
+        try:
+            renderer.upload(scene_to_gpu(scene))
+        finally:
+            renderer.set_hierarchy_build("auto")
+        return renderer.stats()["bvh_depth"], renderer.trace_closest(rays)
+
+    want = {id(s): hits(s, "host") for s in (degenerate, regular)}
+    for scene in (degenerate, degenerate, regular, regular, degenerate):
+        depth, (prim, t) = hits(scene, "auto")
+        want_depth, (want_prim, want_t) = want[id(scene)]
+        assert depth == want_depth
+        assert np.array_equal(prim, want_prim) and np.array_equal(t.view(np.uint32), want_t.view(np.uint32))

@@ -49,8 +49,14 @@ constexpr int kWfRing = kWfLag + 1;
 // Scenes with at least this many primitives build their hierarchy on the device by default. A whole
 // upload with the host / device build (the same tree either way), repeated and into a new context: 512
 // primitives 257 / 328 and 308 / 514 us, 1,024 535 / 390 and 586 / 532, 2,048 1,067 / 442 and 1,116 / 594,
-// 4,000 2,342 / 540 and 2,364 / 749. (A process's first device build also loads its kernels, about 5 ms.)
+// 4,000 2,342 / 540 and 2,364 / 749. The first upload of a process also loads the kernels it launches: 4.1 / 4.7
+// ms at 1,629 primitives, level from about 2,300.
 constexpr size_t kDeviceBuildMin = 1024;
+// A tree with a degenerate leaf is the host's after all, so an attempt on the device is lost: below this
+// size a context whose last build had one goes to the host at once (2,040 spheres, 40 of them coincident:
+// 1.46 ms an upload with the attempt, 1.08 without). From here on the attempt costs little beside the host build, and a scene whose
+// leaf is gone would lose more.
+constexpr size_t kDeviceBuildAlways = 4096;
 // Guide training samples the pool keeps across recording batches (48 bytes each: 768 MiB).
 constexpr uint32_t kGuidePoolSamples = 1u << 24;
 
@@ -122,6 +128,7 @@ struct tc_context {
   // Device hierarchy build (tc_set_hierarchy_build): mode, builder, triangle attribute flags and
   // its status word.
   int build_mode = 0;
+  bool degenerate = false;  // the last hierarchy that an upload built had a degenerate leaf
   bool device_built = false;
   tcb::DeviceBvhBuilder builder;
   DevBuf attr_flags, build_status;
@@ -596,7 +603,8 @@ int tc_upload_scene(tc_context* ctx, const tc_scene_data* sd) {
   // back to the host build, which makes such nodes leaves.
   const size_t n_prims = sd->sphere_count + sd->triangle_count;
   const bool given = sd->bvh_nodes && sd->bvh_node_count;
-  const bool on_device = !given && (ctx->build_mode == 2 || (ctx->build_mode == 0 && n_prims >= kDeviceBuildMin));
+  const size_t device_min = ctx->degenerate ? kDeviceBuildAlways : kDeviceBuildMin;
+  const bool on_device = !given && (ctx->build_mode == 2 || (ctx->build_mode == 0 && n_prims >= device_min));
   bool built = false, unions = true, median_shape = !given;
   uint32_t pair_count = 0, prim_count = 0, depth = 0;
   tcb::DeviceHierarchy dh;
@@ -759,6 +767,7 @@ int tc_upload_scene(tc_context* ctx, const tc_scene_data* sd) {
   ctx->any_attr = any_attr;
   ctx->pair_count = pair_count;
   ctx->median_shape = median_shape;
+  if (!given) ctx->degenerate = !median_shape;
   ctx->device_built = built && on_device;
   ctx->raw_spheres_valid = ctx->device_built;
   ctx->raw_triangles_valid = ctx->device_built || ctx->scene.tri_verts != nullptr;
