@@ -243,7 +243,7 @@ def run_ours(args):
 
     from toaster_b200.native import probe_cache_read
 
-    # The roofline's denominator: L2 read bandwidth (the scene's working set is L2-resident).
+    # L2 read bandwidth, for scale beside the roofline (the scene's working set is L2-resident).
     l2_peak = statistics.median(probe_cache_read(local, 64 << 20, 50) for _ in range(3))
 
     r = GpuRenderer(local)
@@ -325,34 +325,44 @@ def run_ours(args):
         roofline = None
         if cpu is not None:
             # Dominant kernel: the wavefront's trace launches (one per iteration), timed live by the
-            # library's per-phase CUDA events on the render stream. Their algorithmic bytes are the
-            # traversal's node and primitive fetches of every ray the step traced.
+            # library's per-phase CUDA events on the render stream. What binds them is instruction issue
+            # (and the L1 data stage): the committed profile's warp instructions per ray at the live ray
+            # rate, against one instruction per scheduler and clock. Neither L2 nor DRAM is near its rate;
+            # the node and primitive bytes a one-ray-at-a-time traversal of the binary hierarchy would
+            # fetch are given beside, as work done and not as traffic.
             bpr = algorithmic_bytes_per_ray(cpu["counts"])
             trace_ms = statistics.mean(phases["trace_ms"])
             iterations = statistics.mean(phases["wf_iterations"])
-            achieved = bpr * mean_rays / (trace_ms * 1e-3) / 1e9
-            prof = kernel_profile()
-            tpi = prof.get("threads_per_instruction") if prof else None
-            trace_dram = prof.get("dram_bytes_per_ray_trace_kernel") if prof else None
-            roofline = {"bound": "l2", "achieved": achieved, "peak": l2_peak, "unit": "GB/s",
-                        "frac": achieved / l2_peak,
+            rays_per_s = mean_rays / (trace_ms * 1e-3)
+            prof = kernel_profile() or {}
+            per_ray = prof.get("warp_instructions_per_ray_trace_kernel")
+            props = torch.cuda.get_device_properties(local)
+            mhz = clk["sm_mhz"] if clk else None
+            issue_peak = props.multi_processor_count * 4 * mhz * 1e-3 if mhz else None
+            issued = None if per_ray is None else per_ray * rays_per_s / 1e9
+            trace_dram = prof.get("dram_bytes_per_ray_trace_kernel")
+            roofline = {"bound": "issue", "achieved": issued, "peak": issue_peak, "unit": "G warp instructions/s",
+                        "frac": issued / issue_peak if issued and issue_peak else None,
+                        "peak_source": "4 schedulers per SM, one instruction a clock at the SM clock of the timed region",
+                        "warp_instructions_per_ray": per_ray,
+                        "lanes_per_instruction": prof.get("threads_per_instruction"),
+                        "source": prof.get("source"),
                         "traffic": None if trace_dram is None else trace_dram * mean_rays / iterations,
                         "traffic_note": "DRAM bytes per trace launch: ncu's dram__bytes_read + write per ray of "
                                         "the trace launches (8-spp frames of this scene) x rays per launch",
-                        "peak_source": "measured live: L2 read bandwidth of a 64 MiB buffer streamed by every SM "
-                                       "(tc_probe_cache_read, loads bypassing L1)",
-                        "hbm_peak": hbm_peak, "hbm_peak_source": peak_kind, "frac_of_hbm": achieved / hbm_peak,
-                        "issue": None if tpi is None else {
-                            "threads_per_instruction": tpi, "of": 32, "frac": tpi / 32.0,
-                            "source": prof.get("source")},
+                        "dram_gbs": None if trace_dram is None else trace_dram * rays_per_s / 1e9,
+                        "hbm_peak": hbm_peak, "hbm_peak_source": peak_kind,
+                        "binary_traversal_bytes_per_ray": bpr,
+                        "binary_traversal_gbs": bpr * rays_per_s / 1e9,
+                        "l2_read_gbs": l2_peak,
+                        "l2_read_source": "measured live: a 64 MiB buffer streamed by every SM "
+                                          "(tc_probe_cache_read, loads bypassing L1)",
                         "kernel": "wf_trace_wide_kernel (wavefront trace launches)",
-                        "launches_per_step": iterations, "bytes_per_ray": bpr,
-                        "algorithmic_bytes_per_launch": bpr * mean_rays / iterations,
+                        "launches_per_step": iterations,
                         "launch_ms": trace_ms / iterations,
                         "phases_ms_per_step": {k: statistics.mean(phases[k])
                                                for k in ("trace_ms", "logic_ms", "shade_ms")},
-                        "step_kernel_ms": mean_kernel_ms,
-                        "frac_over_whole_step": bpr * mean_rays / (mean_kernel_ms * 1e-3) / 1e9 / l2_peak}
+                        "step_kernel_ms": mean_kernel_ms}
         line = {
             "metric": METRIC,
             "value": value,

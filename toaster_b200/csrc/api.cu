@@ -54,8 +54,8 @@ constexpr int kWfRing = kWfLag + 1;
 constexpr size_t kDeviceBuildMin = 1024;
 // A tree with a degenerate leaf is the host's after all, so an attempt on the device is lost: below this
 // size a context whose last build had one goes to the host at once (2,040 spheres, 40 of them coincident:
-// 1.46 ms an upload with the attempt, 1.08 without). From here on the attempt costs little beside the host build, and a scene whose
-// leaf is gone would lose more.
+// 1.46 ms an upload with the attempt, 1.08 without). From here on the attempt costs little beside the host
+// build, and a scene whose leaf is gone would lose more.
 constexpr size_t kDeviceBuildAlways = 4096;
 // Guide training samples the pool keeps across recording batches (48 bytes each: 768 MiB).
 constexpr uint32_t kGuidePoolSamples = 1u << 24;

@@ -900,8 +900,8 @@ __device__ __forceinline__ void shade_hit(const RenderLaunch& L, const FrameJob&
 // places and the steps in a loop over a switch the instruction cache missed 63 M times on a 4-spp
 // 1280x720 mixed frame (1.5 warps per issue waiting for instructions). With every step once, in order, and
 // the largest shared pieces out of line (59 KB) it misses 27 M times (0.6). At most 80 registers keep 24
-// warps per SM (guided frames, whose step after the inference is longer, run faster with 16 and no
-// spills). Kernel time, before and after: 320x180 x 4 spp of 2,051 primitives 0.65 -> 0.60 ms, mixed
+// warps per SM (guided frames, whose step after the inference is longer, run faster with 20 and no
+// spills; with blocks of 256, which then keep 16, terrain frames lose 6%, 2.57 -> 2.73 ms). Kernel time, before and after: 320x180 x 4 spp of 2,051 primitives 0.65 -> 0.60 ms, mixed
 // scene 640x360 x 4 1.95 -> 1.68 and x 32 12.4 -> 10.5, an animation frame 640x360 x 16 3.92 -> 3.19, the
 // room 480x270 x 4 9.26 -> 8.84, six previews in one launch 3.65 -> 3.45, guided 320x180 x 2 2.05 -> 1.95.
 // The four-wide traversal was tried here too (with and without refills): faster in the room (5.6 ms),
@@ -1426,8 +1426,8 @@ __global__ void __launch_bounds__(kWfBlock, 8) wf_logic_kernel(const WavefrontLa
     // material queues (paths that go on; the shade launch rewrites their state), thread 3 on the
     // work counter for free slots and then on the extension queue for the camera paths that do
     // start (the block's first s_started free slots in block order: items past the frame's last
-    // one start nothing); thread 4 counts the finished paths. Consecutive work items are consecutive pixels of one sample, so a warp's
-    // new rays are neighbours.
+    // one start nothing); thread 4 counts the finished paths. Consecutive work items are consecutive
+    // pixels of one sample, so a warp's new rays are neighbours.
     const int warp = int(threadIdx.x >> 5);
     const unsigned m_mat[3] = {__ballot_sync(0xffffffffu, kind == 0), __ballot_sync(0xffffffffu, kind == 1),
                                __ballot_sync(0xffffffffu, kind == 2)};

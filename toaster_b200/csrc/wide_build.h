@@ -56,7 +56,8 @@ __device__ __forceinline__ void write_lane(LeafPair& p, uint32_t place, const Pr
 __device__ __forceinline__ void wide_children(const PairNode* pairs, const ChildRec& c, ChildRec (&g)[2]) {
   if (c.link & kLeafBit) {
     g[0] = c;
-    g[1] = ChildRec{CUDART_INF_F, CUDART_INF_F, CUDART_INF_F, kLeafBit, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, 0u};
+    g[1] = ChildRec{CUDART_INF_F,  CUDART_INF_F,  CUDART_INF_F,  kLeafBit,
+                    -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, 0u};
   } else {
     g[0] = pairs[c.link].child[0];
     g[1] = pairs[c.link].child[1];

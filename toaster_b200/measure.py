@@ -5,7 +5,7 @@
 
 Reports Mpaths/s, Mrays/s (device-counted extension + shadow rays) and the kernel time per frame
 (CUDA events on the library's stream), for progressive accumulation of `frames` batches of
-`spp` samples per pixel. The scene is uploaded once (hierarchy built on the host).
+`spp` samples per pixel. The scene is uploaded once.
 """
 
 from __future__ import annotations
