@@ -306,6 +306,12 @@ __global__ void trace_closest_kernel(const DevScene s, const float* __restrict__
 // scene), 1,450 -> 904 (room), 432 -> 301 (terrain of 2.1 M triangles), against one thread per ray
 // over the pairs; 65,536 rays: 76 -> 68, 68 -> 65, 214 -> 157 and 93 -> 73; 4,096 rays: 74 -> 49,
 // 64 -> 38, 199 -> 98 and 64 -> 41 us.
+// Rays that hardly diverge gain nothing from the wider step and pay for the refills' set-up: 1,049,600
+// camera rays in image order 178 -> 207, 131 -> 163, 850 -> 874 and 188 -> 193 us, 1,048,576 that miss the
+// scene 15 -> 22 (65,536 camera rays: 65 -> 63, 83 -> 64, 199 -> 142, 57 -> 50). Tried on the mixed scene's
+// 163: refilling only empty warps 157 (random rays 238 -> 425); two to six blocks per resident one 163 to 169
+// (273 to 389); the pair traversal for warps of one origin and nearly one direction, in this kernel 170 to
+// 193 (257 to 270), whose registers it does not have.
 constexpr int kHitsBlock = 128;
 __global__ void __launch_bounds__(kHitsBlock, 8)
     trace_closest_wide_kernel(const __grid_constant__ DevScene s, const float* __restrict__ rays, uint64_t n,
